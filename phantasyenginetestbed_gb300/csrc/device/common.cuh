@@ -15,12 +15,15 @@ namespace phe_gb300 {
 // ------------------------------------------------------------------------------------------------
 // Device scene layout (built on upload from the reference arrays)
 //
-// nodes: 64 B per node, 4 x float4 — bytes 0..47 are the reference fData (child boxes), bytes
-//        48..63 are (child0, child1, count0, count1) with inner children as node indices >= 0 and
-//        leaf children as ~firstSlot (< 0); count is 0 for inner children.
-// tris:  48 B per slot, 3 x float4 — (p0.xyz, endMarker), (e1 = p1 - p0, 0), (e2 = p2 - p0, 0).
-//        e1 and e2 are the exact float subtractions Moller-Trumbore performs first, so storing them
-//        changes no result bit. endMarker is -1 on the last slot of each leaf, else 0.
+// nodes: 64 B per node, two 32-byte halves — (lo.x, lo.y, hi.x, hi.y) of child 0, then of child 1;
+//        (lo.z, hi.z) of child 0, of child 1, then (child0, child1, count0, count1) with inner children
+//        as node indices >= 0 and leaf children as ~firstSlot (< 0); count is 0 for inner children. The
+//        box planes come in the pairs that the packed slab test consumes (traverse.cuh).
+// tris:  48 B per slot, 3 x float4 — (p0.xyz, endMarker), (e2.x, e1.x, e2.y, e1.y), (e2.z, e1.z, 0, 0):
+//        e1 = p1 - p0 and e2 = p2 - p0 interleaved, the operand pairs of the packed triangle test. e1
+//        and e2 are the exact float subtractions Moller-Trumbore performs first, so storing them changes
+//        no result bit. endMarker is -1 on the last slot of each leaf, else 0. (64 B with two 32-byte
+//        loads took 1% longer: more sectors a leaf.)
 // ------------------------------------------------------------------------------------------------
 
 // nodes4 (optional): the same tree collapsed to 4-wide nodes, 128 B each — 6 float4 of child bounds
@@ -54,7 +57,9 @@ struct DeviceScene {
 	uint32_t numTextures, pad;
 	const uint4* nodes8;    // set only while the 8-wide layout is selected (host/wide8.hpp)
 	const float4* leaves8;  // its leaf records
-	uint32_t numNodes8, numLeaves8, pad2[2];
+	uint32_t numNodes8, numLeaves8;
+	float dirLimit;   // a ray direction with components up to this keeps every |det| below 2^126
+	uint32_t pad2;
 };
 static_assert(sizeof(DeviceScene) == 128, "DeviceScene is 128 bytes");
 
@@ -129,6 +134,75 @@ __device__ __forceinline__ float stdmin(float a, float b) { return (b < a) ? b :
 __device__ __forceinline__ float stdmax(float a, float b) { return (a < b) ? b : a; }
 
 // ------------------------------------------------------------------------------------------------
+// Packed FP32 pairs (sm_100 and later): one instruction adds or multiplies two floats, each lane rounded
+// to nearest exactly as the scalar operation. The traversal kernels are bound by instruction issue, so
+// the slab test and the triangle test use them: 258 M against 326 M warp instructions for 1M diffuse
+// rays on 155K triangles, with the loops of traverse.cuh (271 M with a scalar triangle test in them).
+// Products are summed by scalar additions: ptxas contracts a packed product that feeds a packed sum into
+// one fused operation with a single rounding, whatever the rounding modifiers say (measured; a packed
+// sum that feeds a packed product, and a scalar sum of unpacked products, are left alone).
+// ------------------------------------------------------------------------------------------------
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+	f32x2 r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+	f32x2 r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+	f32x2 r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+// (a * b - c * d) of both lanes, lanes swapped: one component of two cross products.
+__device__ __forceinline__ f32x2 cross_swapped(f32x2 a, f32x2 b, f32x2 c, f32x2 d)
+{
+	float p0, p1, n0, n1;
+	unpack2(mul2(a, b), p0, p1);
+	unpack2(mul2(c, d), n0, n1);
+	return pack2(__fsub_rn(p1, n1), __fsub_rn(p0, n0));
+}
+// (ax * bx + ay * by) + az * bz of both lanes.
+__device__ __forceinline__ void dot2(f32x2 ax, f32x2 bx, f32x2 ay, f32x2 by, f32x2 az, f32x2 bz, float& lo, float& hi)
+{
+	float x0, x1, y0, y1, z0, z1;
+	unpack2(mul2(ax, bx), x0, x1);
+	unpack2(mul2(ay, by), y0, y1);
+	unpack2(mul2(az, bz), z0, z1);
+	lo = __fadd_rn(__fadd_rn(x0, y0), z0);
+	hi = __fadd_rn(__fadd_rn(x1, y1), z1);
+}
+// 32 bytes (aligned to 32) of data that no kernel writes, in one load.
+__device__ __forceinline__ void ld32(const void* p, f32x2& a, f32x2& b, f32x2& c, f32x2& d)
+{
+	asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// One slot of `tris` as loaded.
+struct TriSlot {
+	float4 p0;          // p0.xyz, end marker
+	f32x2 ex, ey, ez;   // (e2, e1) per axis
+	__device__ __forceinline__ bool last() const { return p0.w < 0.0f; }
+};
+__device__ __forceinline__ TriSlot load_tri(const float4* __restrict__ tris, uint32_t slot)
+{
+	const float4* p = tris + 3 * (size_t)slot;
+	TriSlot t;
+	t.p0 = __ldg(p);
+	asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(t.ex), "=l"(t.ey) : "l"(p + 1));
+	asm("ld.global.nc.b64 %0, [%1];" : "=l"(t.ez) : "l"(p + 2));
+	return t;
+}
+
+// ------------------------------------------------------------------------------------------------
 // Moller-Trumbore with the reference's absolute determinant epsilon (Intersection.hpp:24-67,
 // RayCastKernel.cu:96-131), on a slot stored as (p0, e1, e2). Returns true on a hit.
 //
@@ -139,22 +213,39 @@ __device__ __forceinline__ float stdmax(float a, float b) { return (a < b) ? b :
 // rejects), while the straight-line form has no branches and overlaps the reciprocal with the other
 // products. f = rn(1 / det) is taken as the correctly rounded reciprocal, the same value as the
 // correctly rounded quotient 1.0f / det.
+//
+// FAST: |det| < 2^126 is known (DeviceScene::dirLimit), so the reciprocal needs no range check: the
+// hardware approximation and one Newton-Raphson step with fused residual, which Markstein (IBM J. Res.
+// Dev. 34, 1990) shows to round correctly up to cases that enumeration settles; all 2^32 floats were
+// compared with __frcp_rn (tests/cpp/reciprocal_test.cu). A |det| below the epsilon is rejected whatever f is.
+// The three instructions and the branch saved are worth 1M diffuse rays on 155K triangles in 314 us
+// instead of 326.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool intersect_tri(float4 a, float4 b, float4 c, f3 o, f3 d, float& t, float& u, float& v)
+__device__ __forceinline__ float reciprocal_in_range(float x)
+{
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+	return __fmaf_rn(r, __fmaf_rn(-x, r, 1.0f), r);
+}
+
+template <bool FAST>
+__device__ __forceinline__ bool intersect_tri(const TriSlot& tri, f3 o, f3 d, float& t, float& u, float& v)
 {
 	const float EPS = 0.00001f;
-	f3 p0 = mk3(a.x, a.y, a.z), e1 = mk3(b.x, b.y, b.z), e2 = mk3(c.x, c.y, c.z);
-	f3 q = cross3(d, e2);
-	float det = dot3(e1, q);
-	f3 s = sub3(o, p0);
-	f3 r = cross3(s, e1);
-	float f = __frcp_rn(det);
-	float uu = __fmul_rn(f, dot3(s, q));
-	float vv = __fmul_rn(f, dot3(d, r));
-	t = __fmul_rn(f, dot3(e2, r));
-	u = uu;
-	v = vv;
-	return !(-EPS < det && det < EPS) && !(uu < 0.0f) && !(vv < 0.0f || __fadd_rn(uu, vv) > 1.0f);
+	const f3 s = mk3(__fsub_rn(o.x, tri.p0.x), __fsub_rn(o.y, tri.p0.y), __fsub_rn(o.z, tri.p0.z));
+	// (r, q) = (s x e1, d x e2), then their products with e and with (d, s)
+	const f32x2 dsx = pack2(d.x, s.x), dsy = pack2(d.y, s.y), dsz = pack2(d.z, s.z);
+	const f32x2 rqx = cross_swapped(dsy, tri.ez, dsz, tri.ey);
+	const f32x2 rqy = cross_swapped(dsz, tri.ex, dsx, tri.ez);
+	const f32x2 rqz = cross_swapped(dsx, tri.ey, dsy, tri.ex);
+	float det, tt, su, dv;
+	dot2(tri.ex, rqx, tri.ey, rqy, tri.ez, rqz, tt, det);   // e2 . r, e1 . q
+	dot2(dsx, rqx, dsy, rqy, dsz, rqz, dv, su);             // d . r, s . q
+	const float f = FAST ? reciprocal_in_range(det) : __frcp_rn(det);
+	u = __fmul_rn(f, su);
+	v = __fmul_rn(f, dv);
+	t = __fmul_rn(f, tt);
+	return !(fabsf(det) < EPS) && !(u < 0.0f) && !(v < 0.0f || __fadd_rn(u, v) > 1.0f);
 }
 
 // ------------------------------------------------------------------------------------------------

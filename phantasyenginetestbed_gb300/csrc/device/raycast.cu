@@ -17,9 +17,12 @@ namespace phe_gb300 {
 
 constexpr int kPlainBlock = 128;
 constexpr int kPersistentBlock = 128;
+// 10 resident blocks of 128 per SM (48 registers): 9 (the compiler's 52 registers) and 8 made 1M diffuse rays
+// 1% and 4% slower, 12 (40 registers, spills) 12%.
+constexpr int kCastMinBlocks = 10;
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kPlainBlock) closest_plain_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays,
+__global__ void __launch_bounds__(kPlainBlock, kCastMinBlocks) closest_plain_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays,
                                                                     phe_ray_hit* __restrict__ hits, uint32_t n,
                                                                     uint32_t* __restrict__ status)
 {
@@ -35,7 +38,7 @@ __global__ void __launch_bounds__(kPlainBlock) closest_plain_kernel(DeviceScene 
 // Persistent warps: each warp takes 32 consecutive rays per atomic fetch (one atomic per warp,
 // lane 0 fetches and broadcasts) until the batch is exhausted.
 template <bool WIDE>
-__global__ void __launch_bounds__(kPersistentBlock) closest_persistent_kernel(DeviceScene s,
+__global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) closest_persistent_kernel(DeviceScene s,
                                                                               const phe_ray_in* __restrict__ rays,
                                                                               phe_ray_hit* __restrict__ hits, uint32_t n,
                                                                               uint32_t* __restrict__ counter,
@@ -60,7 +63,7 @@ __global__ void __launch_bounds__(kPersistentBlock) closest_persistent_kernel(De
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kPersistentBlock) any_persistent_kernel(DeviceScene s,
+__global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) any_persistent_kernel(DeviceScene s,
                                                                           const phe_ray_in* __restrict__ rays,
                                                                           uint8_t* __restrict__ inLight,
                                                                           const uint32_t* __restrict__ scatter, uint32_t n,

@@ -76,12 +76,28 @@ struct ChildRef {
 
 ChildRef binary_child(const std::vector<float4>& dn, uint32_t node, int c)
 {
-	const float* f = reinterpret_cast<const float*>(&dn[(size_t)node * 4]);
+	const float4 xy = dn[(size_t)node * 4 + c], z = dn[(size_t)node * 4 + 2];
 	const int32_t* iv = reinterpret_cast<const int32_t*>(&dn[(size_t)node * 4 + 3]);
 	ChildRef r;
-	for (int k = 0; k < 6; k++) r.box[k] = f[6 * c + k];
+	r.box[0] = xy.x, r.box[1] = xy.y, r.box[3] = xy.z, r.box[4] = xy.w;
+	r.box[2] = c ? z.z : z.x, r.box[5] = c ? z.w : z.y;
 	r.ref = iv[c];
 	return r;
+}
+
+// Largest ray-direction component D for which |det| = |e1 . (d x e2)| <= 6 D E^2 stays below 2^126 (E: the
+// largest edge component of the slots `dt`), with a factor of four to spare for rounding; -1 (no
+// direction) when an edge is not finite.
+float direction_limit(const std::vector<float4>& dt)
+{
+	float e = 0.0f;
+	for (size_t i = 0; i < dt.size(); i += 3)
+		for (float x : {dt[i + 1].x, dt[i + 1].y, dt[i + 1].z, dt[i + 1].w, dt[i + 2].x, dt[i + 2].y}) {
+			if (!std::isfinite(x)) return -1.0f;
+			e = std::max(e, std::fabs(x));
+		}
+	const double limit = 0x1p124 / (6.0 * (double)e * (double)e);
+	return (float)std::min(limit, (double)3.402823466e+38f);
 }
 
 // True when `inner` is a non-inverted box (lo <= hi on every axis) inside `outer`. Then, for a ray
@@ -287,16 +303,17 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	if ((s = check_materials(hm.data(), (uint32_t)hm.size(), nullptr, 0))) return s;
 
 	// Traversal layout: child indices normalised (leaf = ~first), leaf end markers rewritten from
-	// the counts so that leaf loops always stop inside the slot array, triangles as (p0, e1, e2).
+	// the counts so that leaf loops always stop inside the slot array, triangles as p0 and (e1, e2) pairs.
 	std::vector<float4> dn((size_t)numNodes * 4);
 	std::vector<float4> dt((size_t)numSlots * 3);
 	std::vector<uint8_t> used(numSlots, 0);
 	for (uint32_t i = 0; i < numNodes; i++) {
 		const phe_bvh_node& n = hn[i];
 		float4* o = &dn[(size_t)i * 4];
-		o[0] = make_float4(n.fData[0], n.fData[1], n.fData[2], n.fData[3]);
-		o[1] = make_float4(n.fData[4], n.fData[5], n.fData[6], n.fData[7]);
-		o[2] = make_float4(n.fData[8], n.fData[9], n.fData[10], n.fData[11]);
+		const float *b0 = n.fData, *b1 = n.fData + 6;   // lo.xyz, hi.xyz of each child
+		o[0] = make_float4(b0[0], b0[1], b0[3], b0[4]);
+		o[1] = make_float4(b1[0], b1[1], b1[3], b1[4]);
+		o[2] = make_float4(b0[2], b0[5], b1[2], b1[5]);
 		int32_t idx[2], cnt[2];
 		for (int c = 0; c < 2; c++) {
 			int32_t raw = n.iData[c];
@@ -316,9 +333,10 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 		const phe_triangle_vertices& t = hv[i];
 		float e1x = t.v1[0] - t.v0[0], e1y = t.v1[1] - t.v0[1], e1z = t.v1[2] - t.v0[2];
 		float e2x = t.v2[0] - t.v0[0], e2y = t.v2[1] - t.v0[1], e2z = t.v2[2] - t.v0[2];
-		dt[(size_t)i * 3 + 0] = make_float4(t.v0[0], t.v0[1], t.v0[2], 0.0f);
-		dt[(size_t)i * 3 + 1] = make_float4(e1x, e1y, e1z, 0.0f);
-		dt[(size_t)i * 3 + 2] = make_float4(e2x, e2y, e2z, 0.0f);
+		float4* o = &dt[(size_t)i * 3];
+		o[0] = make_float4(t.v0[0], t.v0[1], t.v0[2], 0.0f);
+		o[1] = make_float4(e2x, e1x, e2y, e1y);
+		o[2] = make_float4(e2z, e1z, 0.0f, 0.0f);
 	}
 	// End markers from the leaf ranges of the reachable tree (phe_bvh_validate checked the ranges).
 	{
@@ -415,6 +433,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	sc->maxDepth8 = w8.depth;
 	sc->dev.numNodes8 = sc->numNodes8;
 	sc->dev.numLeaves8 = sc->numLeaves8;
+	sc->dev.dirLimit = direction_limit(dt);
 	sc->dev.numNodes4 = (uint32_t)(dn4.size() / 8);
 	sc->maxDepth4 = depth4;
 	sc->allocation = base;

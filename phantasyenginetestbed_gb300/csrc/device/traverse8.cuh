@@ -195,10 +195,9 @@ __device__ __forceinline__ uint32_t traverse8(const uint4* __restrict__ nodes8, 
 				break;
 			}
 			for (uint32_t j = 0; j < count; j++) {
-				const float4* tp = tris + 3 * (size_t)(first + j);
-				const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+				const TriSlot tri = load_tri(tris, first + j);
 				float t, u, v;
-				if (intersect_tri(ta, tb, tc, r.o, r.d, t, u, v) && r.tMin <= t && t < hit.t) {
+				if (intersect_tri<true>(tri, r.o, r.d, t, u, v) && r.tMin <= t && t < hit.t) {
 					hit.slot = first + j;
 					hit.t = t;
 					hit.u = u;

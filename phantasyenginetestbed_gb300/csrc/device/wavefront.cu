@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kWaveBlock) primary_trace_kernel(DeviceScene s
                                                                    FrameBuffers fb, uint32_t* __restrict__ status)
 {
 	uint32_t err = persistent_trace<false>(s.nodes, s.tris, TraversalBounds{s.numNodes, s.numSlots}, CameraSource{fpp}, HitSink{fb.primaryHits}, fpp->numPixels,
-	                                       fb.counters + kCtrWork0, fb.refill);
+	                                       fb.counters + kCtrWork0, fb.refill, s.dirLimit);
 	if (err) atomicOr(status, err);
 }
 
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kWaveBlock) any_refill_kernel(DeviceScene s, c
                                                                 int refill, uint32_t* __restrict__ status)
 {
 	uint32_t err = persistent_trace<true>(s.nodes, s.tris, TraversalBounds{s.numNodes, s.numSlots}, ArraySource{rays, nullptr}, VisibilitySink{inLight, slots}, *count,
-	                                      work, refill);
+	                                      work, refill, s.dirLimit);
 	if (err) atomicOr(status, err);
 }
 
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kWaveBlock) bounce_trace_kernel(DeviceScene s,
 {
 	uint32_t err = persistent_trace<false>(s.nodes, s.tris, TraversalBounds{s.numNodes, s.numSlots}, ArraySource{fb.bounceRays, fb.sortWindow > 0 ? fb.bouncePerm : nullptr},
 	                                       HitSink{fb.bounceHits},
-	                                       fb.counters[kCtrBounce], fb.counters + kCtrWork1, fb.refill);
+	                                       fb.counters[kCtrBounce], fb.counters + kCtrWork1, fb.refill, s.dirLimit);
 	if (err) atomicOr(status, err);
 }
 
