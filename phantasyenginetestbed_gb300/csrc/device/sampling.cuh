@@ -13,25 +13,62 @@ __device__ __forceinline__ float glsl_mix(float a, float b, float t)
 	return __fadd_rn(__fmul_rn(a, __fsub_rn(1.0f, t)), __fmul_rn(b, t));
 }
 
-// GL_LINEAR with clamp to edge at pixel-space position (px, py) measured from the texel grid origin
-// (texel centres at integer + 0.5) of a W x H image of CH interleaved floats per texel.
-template <int CH>
-__device__ __forceinline__ void bilinear(const float* tex, uint32_t W, uint32_t H, float px, float py, float* out)
+// One axis of GL_LINEAR with clamp to edge: the two texels around pixel-space position p (texel centres at
+// integer + 0.5) of n, and the weight of the second.
+struct LinearAxis {
+	uint32_t i0, i1;
+	float a;
+};
+__device__ __forceinline__ LinearAxis linear_axis(float p, uint32_t n)
 {
-	float fx = __fsub_rn(px, 0.5f), fy = __fsub_rn(py, 0.5f);
-	float x0f = floorf(fx), y0f = floorf(fy);
-	float ax = __fsub_rn(fx, x0f), ay = __fsub_rn(fy, y0f);
-	long x0 = (long)x0f, y0 = (long)y0f, x1 = x0 + 1, y1 = y0 + 1;
-	long Wm = (long)W - 1, Hm = (long)H - 1;
-	x0 = x0 < 0 ? 0 : (x0 > Wm ? Wm : x0);
-	x1 = x1 < 0 ? 0 : (x1 > Wm ? Wm : x1);
-	y0 = y0 < 0 ? 0 : (y0 > Hm ? Hm : y0);
-	y1 = y1 < 0 ? 0 : (y1 > Hm ? Hm : y1);
-	for (int c = 0; c < CH; c++) {
-		float t00 = tex[((size_t)y0 * W + x0) * CH + c], t10 = tex[((size_t)y0 * W + x1) * CH + c];
-		float t01 = tex[((size_t)y1 * W + x0) * CH + c], t11 = tex[((size_t)y1 * W + x1) * CH + c];
-		out[c] = glsl_mix(glsl_mix(t00, t10, ax), glsl_mix(t01, t11, ax), ay);
-	}
+	const float f = __fsub_rn(p, 0.5f), f0 = floorf(f);
+	const int i = (int)f0, m = (int)n - 1;   // images are at most 65536 texels wide and high
+	LinearAxis r;
+	r.a = __fsub_rn(f, f0);
+	r.i0 = (uint32_t)min(max(i, 0), m);
+	r.i1 = (uint32_t)min(max(i == 0x7FFFFFFF ? i : i + 1, 0), m);
+	return r;
 }
+
+__device__ __forceinline__ float2 glsl_mix(float2 a, float2 b, float t) { return make_float2(glsl_mix(a.x, b.x, t), glsl_mix(a.y, b.y, t)); }
+__device__ __forceinline__ float4 glsl_mix(float4 a, float4 b, float t)
+{
+	return make_float4(glsl_mix(a.x, b.x, t), glsl_mix(a.y, b.y, t), glsl_mix(a.z, b.z, t), glsl_mix(a.w, b.w, t));
+}
+
+// One texel of a float2 or float4 image: one load when the image is aligned to its texels (VEC), one per
+// channel for an image that is only aligned to floats.
+template <bool VEC>
+__device__ __forceinline__ float4 ld_texel(const float4* p)
+{
+	if constexpr (VEC) return __ldg(p);
+	const float* f = reinterpret_cast<const float*>(p);
+	return make_float4(__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(f + 3));
+}
+template <bool VEC>
+__device__ __forceinline__ float2 ld_texel(const float2* p)
+{
+	if constexpr (VEC) return __ldg(p);
+	const float* f = reinterpret_cast<const float*>(p);
+	return make_float2(__ldg(f), __ldg(f + 1));
+}
+
+// The four texels of a GL_LINEAR fetch of a float2 or float4 image W texels wide.
+template <bool VEC, class T>
+struct LinearTexels {
+	T t00, t10, t01, t11;
+	__device__ __forceinline__ LinearTexels(const T* __restrict__ tex, uint32_t W, const LinearAxis& x, const LinearAxis& y)
+	{
+		const T *r0 = tex + (size_t)y.i0 * W, *r1 = tex + (size_t)y.i1 * W;
+		t00 = ld_texel<VEC>(r0 + x.i0);
+		t10 = ld_texel<VEC>(r0 + x.i1);
+		t01 = ld_texel<VEC>(r1 + x.i0);
+		t11 = ld_texel<VEC>(r1 + x.i1);
+	}
+	__device__ __forceinline__ T mix(float ax, float ay) const
+	{
+		return glsl_mix(glsl_mix(t00, t10, ax), glsl_mix(t01, t11, ax), ay);
+	}
+};
 
 } // namespace phe_gb300
