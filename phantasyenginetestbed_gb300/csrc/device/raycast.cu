@@ -8,6 +8,7 @@
 // instead of a file-static global reset by a second kernel (RayCastKernel.cu:172-177), so launches
 // on different streams do not share state.
 
+#include <algorithm>
 #include <atomic>
 
 #include "runtime.cuh"
@@ -36,7 +37,20 @@ __global__ void __launch_bounds__(kPlainBlock, kCastMinBlocks) closest_plain_ker
 }
 
 // Persistent warps: each warp takes 32 consecutive rays per atomic fetch (one atomic per warp,
-// lane 0 fetches and broadcasts) until the batch is exhausted.
+// lane 0 fetches and broadcasts) until the batch is exhausted. Without a counter the grid covers the rays and a warp
+// takes the 32 of its own index: a launch of one wave needs no counter cleared before it (2-3 us).
+__device__ __forceinline__ uint32_t next_rays(uint32_t* __restrict__ counter, bool& more)
+{
+	if (!counter) {
+		const uint32_t base = more ? (blockIdx.x * blockDim.x + threadIdx.x) & ~31u : 0xFFFFFFFFu;
+		more = false;
+		return base;
+	}
+	uint32_t base = 0;
+	if ((threadIdx.x & 31u) == 0) base = atomicAdd(counter, 32u);
+	return __shfl_sync(0xffffffffu, base, 0);
+}
+
 template <bool WIDE>
 __global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) closest_persistent_kernel(DeviceScene s,
                                                                               const phe_ray_in* __restrict__ rays,
@@ -45,10 +59,9 @@ __global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) closest_pers
                                                                               uint32_t* __restrict__ status)
 {
 	const uint32_t lane = threadIdx.x & 31u;
+	bool more = true;
 	for (;;) {
-		uint32_t base = 0;
-		if (lane == 0) base = atomicAdd(counter, 32u);
-		base = __shfl_sync(0xffffffffu, base, 0);
+		const uint32_t base = next_rays(counter, more);
 		if (base >= n) break;
 		uint32_t i = base + lane;
 		if (i < n) {
@@ -62,6 +75,67 @@ __global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) closest_pers
 	}
 }
 
+// Launches of few rays (small_cast below): every chunk of rays has a warp from the start, so there is no
+// work counter to clear, and one block an SM spreads the warps over the chip.
+//
+// Such a launch lasts as long as its slowest warp, whose loads no other warp hides: the tree's upper
+// nodes (numTop of them, at most 128 KB) come to shared memory in bulk copies while the rays load, a
+// leaf's triangles are loaded three at a time, and registers are plentiful. 4,096 rays on 10K
+// triangles: closest hit 58 -> 52 us; any hit 51.5 -> 34 us, with 4 rays a warp (below).
+constexpr int kSmallMaxWarps = 16;
+constexpr int kSmallLeaf = 3;
+constexpr int kCopyWaits = 1 << 20;   // bound of the wait for the copy (each try waits some time itself)
+
+__device__ __forceinline__ bool wait_copy(uint32_t barrier)
+{
+	uint32_t done = 0;
+	for (int k = 0; k < kCopyWaits && !done; k++)
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		             : "=r"(done) : "r"(barrier) : "memory");
+	return done != 0;
+}
+
+template <bool ANY>
+__global__ void __launch_bounds__(32 * kSmallMaxWarps, 1)
+small_cast_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays, void* __restrict__ out, const uint32_t* __restrict__ scatter,
+                  uint32_t n, uint32_t numTop, uint32_t raysPerWarp, uint32_t* __restrict__ status)
+{
+	extern __shared__ ulonglong2 topNodes[];
+	__shared__ alignas(8) unsigned long long barrierWord;
+	const uint32_t barrier = (uint32_t)__cvta_generic_to_shared(&barrierWord);
+	if (threadIdx.x == 0) {
+		const uint32_t bytes = numTop * 64u, dst = (uint32_t)__cvta_generic_to_shared(topNodes);
+		asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(barrier));
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+		asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(barrier), "r"(bytes) : "memory");
+		for (uint32_t at = 0; at < bytes; at += 16384u)
+			asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + at),
+			             "l"((const char*)s.nodes + at), "r"(min(16384u, bytes - at)), "r"(barrier)
+			             : "memory");
+	}
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t i = (blockIdx.x + gridDim.x * (threadIdx.x >> 5)) * raysPerWarp + lane;
+	const bool active = lane < raysPerWarp && i < n;
+	RayState r;
+	if (active) r = load_ray(rays, i);
+	__syncthreads();   // the barrier is initialised
+	const bool copied = wait_copy(barrier);
+	if (active) {
+		HitRecord h = empty_hit(r);
+		const TraversalBounds bd{s.numNodes, s.numSlots};
+		const TopNodes nodes{s.nodes, topNodes, copied ? numTop : 0u};
+		const uint32_t err = fast_ray(r, s.dirLimit) ? traverse<true, ANY, 0, kSmallLeaf>(nodes, s.tris, bd, r, h)
+		                                             : traverse<false, ANY, 0, kSmallLeaf>(nodes, s.tris, bd, r, h);
+		if (err) atomicOr(status, err);
+		if (ANY) ((uint8_t*)out)[scatter ? __ldg(scatter + i) : i] = h.slot == ~0u ? 1 : 0;
+		else store_hit((phe_ray_hit*)out, i, r, h);
+	}
+	if (!copied) {   // the copy still writes this block's shared memory
+		if (threadIdx.x == 0) atomicOr(status, kErrTopCopy);
+		wait_copy(barrier);
+	}
+}
+
 template <bool WIDE>
 __global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) any_persistent_kernel(DeviceScene s,
                                                                           const phe_ray_in* __restrict__ rays,
@@ -71,10 +145,9 @@ __global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) any_persiste
                                                                           uint32_t* __restrict__ status)
 {
 	const uint32_t lane = threadIdx.x & 31u;
+	bool more = true;
 	for (;;) {
-		uint32_t base = 0;
-		if (lane == 0) base = atomicAdd(counter, 32u);
-		base = __shfl_sync(0xffffffffu, base, 0);
+		const uint32_t base = next_rays(counter, more);
 		if (base >= n) break;
 		uint32_t i = base + lane;
 		if (i < n) {
@@ -117,6 +190,42 @@ static phe_status check_cast_args(const phe_scene* scene, const void* rays, cons
 	return PHE_OK;
 }
 
+// Queues a launch of few rays on binary nodes (*done) or leaves it to the caller.
+//
+// Closest hit keeps 32 consecutive rays a warp: which of a duplicated triangle's slots a ray reports depends on
+// when its warp turns to leaves, so other warps would report other duplicates. Any hit has no such
+// choice and takes as few rays a warp (4 to 32) as fill the resident warps: fewer lanes wait for one another.
+// Where the lines lie (155K triangles, us a call, small / the kernels above): closest hit 4,096 surface rays 75 / 79,
+// 65,536 93 / 96, on 2M triangles 131 / 136 and 233 / 230; any hit 37 / 62 at 4,096, 68 / 76 at the 77,824 rays that
+// 16 warps an SM hold.
+constexpr uint32_t kSmallClosestRays = 49152;
+template <bool ANY>
+static phe_status small_cast(const phe_scene* scene, const phe_ray_in* rays, void* out, const uint32_t* scatter, uint32_t n,
+                             cudaStream_t stream, bool* done)
+{
+	*done = false;
+	if (scene->dev.nodes4 || scene->dev.nodes8 || (!ANY && n > kSmallClosestRays)) return PHE_OK;
+	DeviceInfo* d = nullptr;
+	if (phe_status st = device_info(&d)) return st;
+	const uint32_t maxWarps = (uint32_t)d->numSMs * kSmallMaxWarps;
+	uint32_t perWarp = ANY ? 4u : 32u;
+	while (perWarp < 32u && (n - 1) / perWarp >= maxWarps) perWarp *= 2;
+	if ((n - 1) / perWarp >= maxWarps) return PHE_OK;
+	const uint32_t warps = (n - 1) / perWarp + 1, grid = std::min(warps, (uint32_t)d->numSMs), perBlock = (warps - 1) / grid + 1;
+	const size_t smem = (size_t)scene->dev.numTop * 64u;
+	auto kernel = small_cast_kernel<ANY>;
+	static std::atomic<uint64_t> sized{0};   // devices on which the kernel may use that much shared memory
+	if (!(sized.load(std::memory_order_relaxed) >> d->device & 1u)) {
+		PHE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kTopNodes * 64u)),
+		             "small_cast_kernel shared memory");
+		sized.fetch_or(uint64_t(1) << d->device, std::memory_order_relaxed);
+	}
+	kernel<<<grid, 32 * perBlock, smem, stream>>>(scene->dev, rays, out, scatter, n, scene->dev.numTop, perWarp, scene->status);
+	PHE_CUDA_TRY(cudaGetLastError(), "small_cast_kernel launch");
+	*done = true;
+	return PHE_OK;
+}
+
 } // namespace phe_gb300
 
 using namespace phe_gb300;
@@ -128,6 +237,8 @@ extern "C" phe_status phe_cast_closest_plain(const phe_scene* scene, const phe_r
 	if (st) return st;
 	if (((uintptr_t)hits & 15u) != 0) return fail(PHE_ERR_INVALID_ARGUMENT, "hit buffer must be 16-byte aligned");
 	if (n == 0) return PHE_OK;
+	bool done = false;
+	if ((st = small_cast<false>(scene, rays, hits, nullptr, n, (cudaStream_t)stream, &done)) || done) return st;
 	uint32_t grid = (n + kPlainBlock - 1) / kPlainBlock;
 	auto kernel = (scene->dev.nodes4 || scene->dev.nodes8) ? closest_plain_kernel<true> : closest_plain_kernel<false>;
 	kernel<<<grid, kPlainBlock, stack_smem_bytes(kPlainBlock), (cudaStream_t)stream>>>(scene->dev, rays, hits, n,
@@ -143,15 +254,17 @@ extern "C" phe_status phe_cast_closest(const phe_scene* scene, const phe_ray_in*
 	if (st) return st;
 	if (((uintptr_t)hits & 15u) != 0) return fail(PHE_ERR_INVALID_ARGUMENT, "hit buffer must be 16-byte aligned");
 	if (n == 0) return PHE_OK;
+	bool done = false;
+	if ((st = small_cast<false>(scene, rays, hits, nullptr, n, (cudaStream_t)stream, &done)) || done) return st;
 	if (n > kMaxPersistentRays) return fail(PHE_ERR_TOO_LARGE, "phe_cast_closest: at most %u rays per launch", kMaxPersistentRays);
 	const bool wide = scene->dev.nodes4 || scene->dev.nodes8;
 	auto kernel = wide ? closest_persistent_kernel<true> : closest_persistent_kernel<false>;
 	int grid = 0;
 	if ((st = persistent_grid(wide ? 2 : 0, (const void*)kernel, &grid))) return st;
 	uint32_t maxGrid = (n + kPersistentBlock - 1) / kPersistentBlock;
-	if ((uint32_t)grid > maxGrid) grid = (int)maxGrid;
 	uint32_t* counter = nullptr;
-	if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
+	if ((uint32_t)grid >= maxGrid) grid = (int)maxGrid;   // one wave: no counter
+	else if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
 	kernel<<<grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream>>>(scene->dev, rays, hits,
 	                                                                                             n, counter,
 	                                                                                             scene->status);
@@ -165,15 +278,17 @@ extern "C" phe_status phe_cast_any(const phe_scene* scene, const phe_ray_in* ray
 	phe_status st = check_cast_args(scene, rays, inLight);
 	if (st) return st;
 	if (n == 0) return PHE_OK;
+	bool done = false;
+	if ((st = small_cast<true>(scene, rays, inLight, scatter, n, (cudaStream_t)stream, &done)) || done) return st;
 	if (n > kMaxPersistentRays) return fail(PHE_ERR_TOO_LARGE, "phe_cast_any: at most %u rays per launch", kMaxPersistentRays);
 	const bool wide = scene->dev.nodes4 || scene->dev.nodes8;
 	auto kernel = wide ? any_persistent_kernel<true> : any_persistent_kernel<false>;
 	int grid = 0;
 	if ((st = persistent_grid(wide ? 3 : 1, (const void*)kernel, &grid))) return st;
 	uint32_t maxGrid = (n + kPersistentBlock - 1) / kPersistentBlock;
-	if ((uint32_t)grid > maxGrid) grid = (int)maxGrid;
 	uint32_t* counter = nullptr;
-	if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
+	if ((uint32_t)grid >= maxGrid) grid = (int)maxGrid;   // one wave: no counter
+	else if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
 	kernel<<<grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream>>>(scene->dev, rays,
 	                                                                                             inLight, scatter, n,
 	                                                                                             counter,

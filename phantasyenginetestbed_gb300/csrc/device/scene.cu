@@ -7,7 +7,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "../host/wide8.hpp"
@@ -83,6 +85,50 @@ ChildRef binary_child(const std::vector<float4>& dn, uint32_t node, int c)
 	r.box[2] = c ? z.z : z.x, r.box[5] = c ? z.w : z.y;
 	r.ref = iv[c];
 	return r;
+}
+
+// Moves the tree's upper nodes to the front of the traversal layout `dn`: the kTopNodes with the largest
+// boxes, taken best first from the root (a child never precedes its parent, and the likelier a random
+// ray visits a node, the earlier it comes). A launch of few rays copies them to shared memory. The
+// others keep their order. Child references follow; nothing else depends on a node's index.
+uint32_t move_top_nodes(std::vector<float4>& dn, uint32_t numNodes)
+{
+	auto area = [](const ChildRef& c) {
+		const float x = c.box[3] - c.box[0], y = c.box[4] - c.box[1], z = c.box[5] - c.box[2];
+		return x * y + y * z + z * x;
+	};
+	std::vector<uint32_t> order;
+	std::vector<uint8_t> moved(numNodes, 0);
+	order.reserve(numNodes);
+	std::priority_queue<std::pair<float, uint32_t>> open;
+	open.push({std::numeric_limits<float>::infinity(), 0u});
+	while (!open.empty() && order.size() < kTopNodes) {
+		const uint32_t n = open.top().second;
+		open.pop();
+		moved[n] = 1;
+		order.push_back(n);
+		for (int c = 0; c < 2; c++) {
+			const ChildRef ch = binary_child(dn, n, c);
+			if (ch.ref >= 0) {
+				const float a = area(ch);
+				open.push({std::isnan(a) ? 0.0f : a, (uint32_t)ch.ref});
+			}
+		}
+	}
+	const uint32_t numTop = (uint32_t)order.size();
+	for (uint32_t n = 0; n < numNodes; n++)
+		if (!moved[n]) order.push_back(n);
+	std::vector<uint32_t> at(numNodes);
+	for (uint32_t k = 0; k < numNodes; k++) at[order[k]] = k;
+	std::vector<float4> out(dn.size());
+	for (uint32_t k = 0; k < numNodes; k++) {
+		std::copy_n(&dn[(size_t)order[k] * 4], 4, &out[(size_t)k * 4]);
+		int32_t* iv = reinterpret_cast<int32_t*>(&out[(size_t)k * 4 + 3]);
+		for (int c = 0; c < 2; c++)
+			if (iv[c] >= 0) iv[c] = (int32_t)at[iv[c]];
+	}
+	dn.swap(out);
+	return numTop;
 }
 
 // Largest ray-direction component D for which |det| = |e1 . (d x e2)| <= 6 D E^2 stays below 2^126 (E: the
@@ -305,7 +351,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	// Traversal layout: child indices normalised (leaf = ~first), leaf end markers rewritten from
 	// the counts so that leaf loops always stop inside the slot array, triangles as p0 and (e1, e2) pairs.
 	std::vector<float4> dn((size_t)numNodes * 4);
-	std::vector<float4> dt((size_t)numSlots * 3);
+	std::vector<float4> dt(((size_t)numSlots + kTriPadding) * 3);
 	std::vector<uint8_t> used(numSlots, 0);
 	for (uint32_t i = 0; i < numNodes; i++) {
 		const phe_bvh_node& n = hn[i];
@@ -373,6 +419,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 		w8.leaves.clear();
 	}
 
+	const uint32_t numTop = move_top_nodes(dn, numNodes);
 	size_t nodeBytes = align256(dn.size() * sizeof(float4));
 	size_t node4Bytes = align256(dn4.size() * sizeof(float4));
 	size_t node8Bytes = align256(w8.nodes.size() * sizeof(uint32_t));
@@ -434,6 +481,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	sc->dev.numNodes8 = sc->numNodes8;
 	sc->dev.numLeaves8 = sc->numLeaves8;
 	sc->dev.dirLimit = direction_limit(dt);
+	sc->dev.numTop = numTop;
 	sc->dev.numNodes4 = (uint32_t)(dn4.size() / 8);
 	sc->maxDepth4 = depth4;
 	sc->allocation = base;

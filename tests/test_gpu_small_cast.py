@@ -1,0 +1,59 @@
+"""Launches of few rays (their own kernel, then one wave without a work counter) give the bits of the same rays
+in a large launch, at the sizes where the kernel, its rays per warp and its blocks change."""
+import functools
+
+import numpy as np
+import pytest
+
+import phantasyenginetestbed_gb300 as P
+from oracle import oracle as O
+from tests.helpers import built_scene, device_empty, from_device, random_rays, to_device
+
+pytestmark = pytest.mark.gpu
+N = 400_000   # more than one wave of any device of 152 SMs
+
+
+@functools.lru_cache(maxsize=None)
+def _large(name):
+    """The scene, N rays on the device and their results in one launch of the persistent kernels."""
+    import torch
+    if name == "one_leaf":
+        b = P.build_sbvh(np.array([[0, 0, 0, 1, 0, 0, 0, 1, 0], [0, 0, 0.5, 1, 0, 0.5, 0, 1, 0.5]], np.float32))
+        k = 1.0
+    else:
+        s, b = built_scene(name)
+        k = s.scale
+    scene = P.Scene(b.nodes, b.verts)
+    rays = random_rays(N, [0, 0, 0.01 * k], [k, k, 0.3 * k], 21)
+    d_rays = to_device(rays)
+    hits, vis = device_empty(N, P.RAY_HIT_DTYPE), device_empty(N, np.uint8)
+    P.cast_closest(scene, d_rays, hits, N)
+    P.cast_any(scene, d_rays, vis, N)
+    torch.cuda.synchronize()
+    return b, scene, rays, d_rays, from_device(hits, P.RAY_HIT_DTYPE), from_device(vis, np.uint8)
+
+
+@pytest.mark.parametrize("name", ["c1_64_100", "c2_256_2000", "one_leaf"])
+@pytest.mark.parametrize("n", [1, 31, 33, 152 * 32 + 1, 152 * 16 * 4, 152 * 16 * 4 + 1, 152 * 16 * 8 + 1, 49152, 49153,
+                               152 * 16 * 32, 152 * 16 * 32 + 1, 152 * 1280, 152 * 1280 + 1])
+def test_small_launches_give_the_large_launch(name, n):
+    import torch
+    b, scene, rays, d_rays, hits, vis = _large(name)
+    for cast in (P.cast_closest, P.cast_closest_plain):
+        out = device_empty(n, P.RAY_HIT_DTYPE)
+        cast(scene, d_rays, out, n)
+        torch.cuda.synchronize()
+        assert np.array_equal(from_device(out, np.uint8), hits[:n].view(np.uint8))
+    order = np.random.default_rng(n).permutation(n).astype(np.uint32)
+    for scatter in (None, order):
+        out = torch.full((n + 16,), 7, dtype=torch.uint8, device="cuda")
+        P.cast_any(scene, d_rays, out, n, scatter=None if scatter is None else to_device(scatter))
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert np.array_equal(got[:n] if scatter is None else got[:n][order], vis[:n])
+        assert np.all(got[n:] == 7)
+    assert scene.status() == 0
+    if n == 33:
+        assert np.array_equal(vis[:20000], O.any_rays(b.nodes, b.verts, rays[:20000]))
+        orc = O.cast_rays(b.nodes, b.verts, rays[:20000], mode=O.MODE_GPU)
+        assert O.compare_closest(hits[:20000], orc, rays[:20000], b.slot_to_tri, b.verts)["ok"]
