@@ -34,14 +34,11 @@
 namespace phe_gb300 {
 
 constexpr int kWaveBlock = 128;
-// Resident blocks per SM asked of the compiler for the fused traversal + shading kernels: caps them
-// at 64 registers (32 warps per SM instead of 20-24). The spills this costs sit in the shading code;
-// measured on GB300 at 1080p: 8 blocks 0.893 ms per frame, 9 0.926, 10 0.915, 12 0.959, uncapped
-// (88-92 registers) 0.970. With the branch-free triangle test (fewer live values) the bounce kernel,
-// whose incoherent rays wait longest on node fetches, gains from more resident warps while the
-// primary kernel does not: bounce pass 0.369 ms at 10 blocks (48 registers) vs 0.376 at 8 and 0.377
-// at 12; primary 0.242 ms at 8 vs 0.245 at 9 or 10.
-constexpr int kWaveMinBlocks = 8;
+// Resident blocks per SM asked of the compiler for the fused traversal + shading kernels: 10 caps them at
+// 48 registers (40 warps per SM). The spills this costs sit in the shading code; a 1080p frame with the
+// primary kernel at 7 / 8 / 9 / 10 blocks took 0.657 / 0.652 / 0.650 / 0.645 ms, with the bounce kernel at 8 / 9 /
+// 10 / 12 blocks 0.664 / 0.658 / 0.652 / 0.658.
+constexpr int kWaveMinBlocks = 10;
 constexpr int kBounceMinBlocks = 10;
 const size_t kStackSmem = stack_smem_bytes(kWaveBlock);   // dynamic shared memory of the traversal kernels
 
