@@ -413,7 +413,7 @@ phe_status phe_renderer_set_shadow_schedule(phe_renderer* renderer, int schedule
  * replayed). Enabling resets the totals. kernel_times returns the summed milliseconds per frame kernel
  * (in launch order, `numKernels` of them) and the number of frames timed. */
 phe_status phe_renderer_set_kernel_timing(phe_renderer* renderer, int enable);
-/* Bytes copied host -> device per frame (the frame parameter block: camera, jitter, lights). */
+/* Bytes copied host -> device per frame (the frame parameter block: camera, jitter, lights; cleared counters). */
 uint32_t phe_renderer_frame_param_bytes(void);
 phe_status phe_renderer_kernel_times(phe_renderer* renderer, double msTotal[8], uint32_t* numKernels, uint32_t* frames);
 /* Frames in flight (no reference counterpart; the reference renders and presents one frame at a time).

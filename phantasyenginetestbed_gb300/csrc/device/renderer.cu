@@ -37,7 +37,7 @@ struct phe_renderer {
 	FrameBuffers fb1{};                  // slot 1: fb with its per-frame buffers replaced
 	void* allocation1 = nullptr;
 	int inFlight = 1;
-	FrameParamsDev* dParams1 = nullptr;  // parameters of slot 1
+	FrameHeadDev* dParams1 = nullptr;    // parameters and counters of slot 1
 	cudaStream_t travStream[2] = {}, resolveStream = nullptr;
 	cudaEvent_t callEvent = nullptr;     // the caller's work before a render
 	cudaEvent_t travDone[2] = {}, resolveDone[2] = {};
@@ -54,13 +54,13 @@ struct phe_renderer {
 	cudaEvent_t partFork = nullptr, partJoin[kMaxFrameParts] = {};
 	void* partAlloc[kMaxFrameParts] = {};
 	FrameBuffers partFb[kMaxFrameParts] = {};
-	FrameParamsDev* partParams[kMaxFrameParts] = {};   // parameters of parts 2.. (part 1: dParams1)
+	FrameHeadDev* partParams[kMaxFrameParts] = {};   // parameters and counters of parts 2.. (part 1: dParams1)
 	// Latency recording of frames in flight: (start, end) event pairs, drained by frame_latencies.
 	bool recordLatency = false;
 	std::vector<cudaEvent_t> latencyPool;
 	std::vector<std::pair<cudaEvent_t, cudaEvent_t>> latencyPending;
-	FrameParamsDev* dParams = nullptr;
-	FrameParamsDev* hParams = nullptr;   // pinned staging ring of kParamSlots
+	FrameHeadDev* dParams = nullptr;
+	FrameHeadDev* hParams = nullptr;     // pinned staging ring of kParamSlots (the counters stay 0)
 	cudaEvent_t paramEvents[8] = {};     // last copy out of each staging slot
 	uint32_t paramSlot = 0;
 	size_t capacityP = 0, capacityL = 0; // frame buffers are kept while a resolution fits
@@ -115,7 +115,7 @@ static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Buffers and parameters of part j of a split frame (part 0: the renderer's own).
 static const FrameBuffers& part_fb(const phe_renderer* r, uint32_t j) { return j == 0 ? r->fb : j == 1 ? r->fb1 : r->partFb[j]; }
-static FrameParamsDev* part_params(const phe_renderer* r, uint32_t j)
+static FrameHeadDev* part_params(const phe_renderer* r, uint32_t j)
 {
 	return j == 0 ? r->dParams : j == 1 ? r->dParams1 : r->partParams[j];
 }
@@ -162,7 +162,7 @@ static void free_buffers(phe_renderer* r)
 
 // Per-frame buffers of one slot: everything a frame's traversal writes and its resolve reads. Sizes
 // for P pixels and L lights, in carving order.
-static const int kPerFrameParts = 12;
+static const int kPerFrameParts = 11;
 static void per_frame_sizes(size_t P, size_t L, size_t sizes[kPerFrameParts])
 {
 	const size_t LP = P * L;
@@ -175,7 +175,6 @@ static void per_frame_sizes(size_t P, size_t L, size_t sizes[kPerFrameParts])
 		P * sizeof(uint32_t),             // bouncePixel
 		P * sizeof(float4),               // bounceThroughput
 		P * sizeof(float),                // roughness
-		kNumCounters * sizeof(uint32_t),  // counters
 		P * sizeof(phe_ray_hit),          // primaryHits
 		P * sizeof(phe_ray_hit),          // bounceHits
 		P * sizeof(uint32_t),             // bouncePerm
@@ -191,8 +190,9 @@ static size_t per_frame_bytes(size_t P, size_t L)
 	return total;
 }
 
-// Points fb's per-frame buffers into `base` (per_frame_bytes(P, L) bytes); returns the end.
-static char* carve_per_frame(char* base, size_t P, size_t L, FrameBuffers& fb)
+// Points fb's per-frame buffers into `base` (per_frame_bytes(P, L) bytes) and its counters to `head`; returns
+// the end.
+static char* carve_per_frame(char* base, size_t P, size_t L, FrameHeadDev* head, FrameBuffers& fb)
 {
 	size_t sizes[kPerFrameParts];
 	per_frame_sizes(P, L, sizes);
@@ -206,10 +206,10 @@ static char* carve_per_frame(char* base, size_t P, size_t L, FrameBuffers& fb)
 	fb.bouncePixel = (uint32_t*)take(5);
 	fb.bounceThroughput = (float4*)take(6);
 	fb.roughness = (float*)take(7);
-	fb.counters = (uint32_t*)take(8);
-	fb.primaryHits = (phe_ray_hit*)take(9);
-	fb.bounceHits = (phe_ray_hit*)take(10);
-	fb.bouncePerm = (uint32_t*)take(11);
+	fb.primaryHits = (phe_ray_hit*)take(8);
+	fb.bounceHits = (phe_ray_hit*)take(9);
+	fb.bouncePerm = (uint32_t*)take(10);
+	fb.counters = head->counters;   // an address on the device
 	return p;
 }
 
@@ -227,13 +227,13 @@ static void make_fb1(phe_renderer* r)
 {
 	if (r->allocation1) {
 		r->fb1 = r->fb;
-		carve_per_frame((char*)r->allocation1, r->capacityP, r->capacityL, r->fb1);
+		carve_per_frame((char*)r->allocation1, r->capacityP, r->capacityL, r->dParams1, r->fb1);
 		if (r->frameParts >= 2) share_pixels(r, r->fb1);
 	}
 	for (int j = 2; j < kMaxFrameParts; j++)
 		if (r->partAlloc[j]) {
 			r->partFb[j] = r->fb;
-			carve_per_frame((char*)r->partAlloc[j], r->capacityP, r->capacityL, r->partFb[j]);
+			carve_per_frame((char*)r->partAlloc[j], r->capacityP, r->capacityL, r->partParams[j], r->partFb[j]);
 			share_pixels(r, r->partFb[j]);
 		}
 }
@@ -256,6 +256,7 @@ static phe_status allocate_slot1(phe_renderer* r)
 		return cuda_fail(e, "cudaMalloc(frame buffers of the second frame in flight)");
 	}
 	make_fb1(r);
+	if (phe_status st = clear_new(r->dParams1, sizeof(FrameHeadDev))) return st;
 	return clear_new(r->allocation1, bytes);
 }
 
@@ -272,6 +273,7 @@ static phe_status allocate_parts(phe_renderer* r)
 			return cuda_fail(e, "cudaMalloc(ray queues of a frame part)");
 		}
 		make_fb1(r);
+		if (phe_status st = clear_new(r->partParams[j], sizeof(FrameHeadDev))) return st;
 		if (phe_status st = clear_new(r->partAlloc[j], bytes)) return st;
 	}
 	return PHE_OK;
@@ -307,7 +309,7 @@ static phe_status prepare_parts(phe_renderer* r, int parts)
 		if (!r->partJoin[j])
 			PHE_CUDA_TRY(cudaEventCreateWithFlags(&r->partJoin[j], cudaEventDisableTiming), "create part event");
 		if (j >= 2 && !r->partParams[j])
-			PHE_CUDA_TRY(cudaMalloc(&r->partParams[j], sizeof(FrameParamsDev)), "allocate part parameters");
+			PHE_CUDA_TRY(cudaMalloc(&r->partParams[j], sizeof(FrameHeadDev)), "allocate part parameters");
 	}
 	phe_status st = allocate_slot1(r);
 	if (!st) st = allocate_parts(r);
@@ -352,7 +354,7 @@ static phe_status allocate(phe_renderer* r, uint32_t resX, uint32_t resY, uint32
 	cudaError_t e = cudaMalloc(&base, total);
 	if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(frame buffers)");
 	FrameBuffers& fb = r->fb;
-	char* p = carve_per_frame(base, P, L, fb);
+	char* p = carve_per_frame(base, P, L, r->dParams, fb);
 	auto take = [&](size_t i) { char* q = p; p += align256(shared[i]); return q; };
 	fb.rawColor = (float4*)take(0);
 	fb.history[0] = (float4*)take(1);
@@ -370,6 +372,7 @@ static phe_status allocate(phe_renderer* r, uint32_t resX, uint32_t resY, uint32
 	r->resX = resX;
 	r->resY = resY;
 	r->numLights = numLights;
+	if (phe_status st = clear_new(r->dParams, sizeof(FrameHeadDev))) return st;
 	if (phe_status st = clear_new(base, total)) return st;
 	r->parity = 0;
 	if (r->inFlight == 2 || r->frameParts >= 2) {
@@ -485,9 +488,9 @@ extern "C" phe_status phe_renderer_create(phe_renderer** out)
 	phe_status st = device_info(&d);
 	if (st) return st;
 	phe_renderer* r = new phe_renderer();
-	cudaError_t e = cudaMalloc(&r->dParams, sizeof(FrameParamsDev));
-	if (e == cudaSuccess) e = cudaMalloc(&r->dParams1, sizeof(FrameParamsDev));
-	if (e == cudaSuccess) e = cudaMallocHost(&r->hParams, sizeof(FrameParamsDev) * kParamSlots);
+	cudaError_t e = cudaMalloc(&r->dParams, sizeof(FrameHeadDev));
+	if (e == cudaSuccess) e = cudaMalloc(&r->dParams1, sizeof(FrameHeadDev));
+	if (e == cudaSuccess) e = cudaMallocHost(&r->hParams, sizeof(FrameHeadDev) * kParamSlots);
 	for (uint32_t i = 0; i < kParamSlots && e == cudaSuccess; i++)
 		e = cudaEventCreateWithFlags(&r->paramEvents[i], cudaEventDisableTiming);
 	if (e != cudaSuccess) {
@@ -497,7 +500,7 @@ extern "C" phe_status phe_renderer_create(phe_renderer** out)
 		delete r;
 		return cuda_fail(e, "allocate frame parameters");
 	}
-	std::memset(r->hParams, 0, sizeof(FrameParamsDev) * kParamSlots);
+	std::memset(r->hParams, 0, sizeof(FrameHeadDev) * kParamSlots);
 	// No stream of its own yet: CUDA maps streams onto a few hardware queues in creation order, so
 	// streams that sit unused (the side stream of a schedule not chosen) would make the streams of
 	// concurrent renderers share queues and wait on each other. The side stream comes with the
@@ -742,8 +745,11 @@ extern "C" phe_status phe_renderer_reset_taa(phe_renderer* r, void* stream)
 		st = guard_side(r, side, (cudaStream_t)stream);
 		if (st) return st;
 	}
-	PHE_CUDA_TRY(cudaMemsetAsync(r->fb.history[0], 0, P * sizeof(float4), (cudaStream_t)stream), "reset TAA");
-	PHE_CUDA_TRY(cudaMemsetAsync(r->fb.history[1], 0, P * sizeof(float4), (cudaStream_t)stream), "reset TAA");
+	// The two histories follow one another when the buffers were allocated for this resolution: one memset.
+	const bool adjacent = r->fb.history[1] == r->fb.history[0] + P;
+	PHE_CUDA_TRY(cudaMemsetAsync(r->fb.history[0], 0, (adjacent ? 2 : 1) * P * sizeof(float4), (cudaStream_t)stream), "reset TAA");
+	if (!adjacent)
+		PHE_CUDA_TRY(cudaMemsetAsync(r->fb.history[1], 0, P * sizeof(float4), (cudaStream_t)stream), "reset TAA");
 	r->hasPrevCam = false;
 	r->velZero[0] = r->velZero[1] = r->velZero[2] = true;
 	return PHE_OK;
@@ -774,14 +780,14 @@ extern "C" phe_status phe_renderer_ray_totals_async(const phe_renderer* r, uint6
 static phe_status launch_whole_or_split(phe_renderer* r, cudaStream_t s, uint32_t parts, const uint32_t* n)
 {
 	if (parts == 1)
-		return launch_frame(r->scene, r->dParams, r->fb, r->resX, r->resY, s, nullptr, r->fused, r->shadowSchedule,
+		return launch_frame(r->scene, &r->dParams->params, r->fb, r->resX, r->resY, s, nullptr, r->fused, r->shadowSchedule,
 		                    &r->streams);
 	PHE_CUDA_TRY(cudaEventRecord(r->partFork, s), "fork frame parts");
 	for (uint32_t j = 1; j < parts; j++)
 		PHE_CUDA_TRY(cudaStreamWaitEvent(r->partStream[j], r->partFork, 0), "fork frame parts");
 	for (uint32_t j = 0; j < parts; j++) {
 		cudaStream_t ps = j ? r->partStream[j] : s;
-		phe_status st = launch_frame(r->scene, part_params(r, j), part_fb(r, j), r->resX, r->resY, ps, nullptr, r->fused,
+		phe_status st = launch_frame(r->scene, &part_params(r, j)->params, part_fb(r, j), r->resX, r->resY, ps, nullptr, r->fused,
 		                             r->shadowSchedule, nullptr, kFrameAll, n[j]);
 		if (st) return st;
 		if (j) PHE_CUDA_TRY(cudaEventRecord(r->partJoin[j], ps), "join frame parts");
@@ -815,7 +821,8 @@ extern "C" phe_status phe_renderer_render(phe_renderer* r, const phe_sphere_ligh
 	const bool pipelined = r->inFlight == 2 && !r->timing;
 	const uint32_t j = pipelined ? r->nextSlot : 0;
 	const FrameBuffers& fb = j ? r->fb1 : r->fb;
-	FrameParamsDev* dParams = j ? r->dParams1 : r->dParams;
+	FrameHeadDev* dHead = j ? r->dParams1 : r->dParams;
+	const FrameParamsDev* dParams = &dHead->params;   // an address on the device
 	cudaStream_t X = pipelined ? r->travStream[j] : s;   // traversal kernels
 	cudaStream_t R = pipelined ? r->resolveStream : s;   // resolve + TAA
 	// A split frame: part j takes the tile rows r with r % parts == j, part 0 on `s`, the others on their
@@ -843,7 +850,7 @@ extern "C" phe_status phe_renderer_render(phe_renderer* r, const phe_sphere_ligh
 	uint32_t slot = r->paramSlot;
 	r->paramSlot = (slot + 1) % kParamSlots;
 	PHE_CUDA_TRY(cudaEventSynchronize(r->paramEvents[slot]), "wait for a free parameter slot");
-	FrameParamsDev& fp = r->hParams[slot];
+	FrameParamsDev& fp = r->hParams[slot].params;
 	// Camera motion: this frame writes the next entry of the velocity ring and reads the previous
 	// frame's; a camera equal to the previous one has velocity 0 (nothing written or read).
 	const uint32_t outSide = r->parity ^ 1u;
@@ -872,18 +879,18 @@ extern "C" phe_status phe_renderer_render(phe_renderer* r, const phe_sphere_ligh
 	phe_status gst = guard_velocity(r, vOut, X);   // the traversal rewrites this velocity buffer
 	if (!gst) gst = guard_side(r, outSide, R);     // the resolve rewrites this colour / history side
 	if (gst) return gst;
-	PHE_CUDA_TRY(cudaMemcpyAsync(dParams, &fp, sizeof(FrameParamsDev), cudaMemcpyHostToDevice, X),
+	PHE_CUDA_TRY(cudaMemcpyAsync(dHead, &r->hParams[slot], sizeof(FrameHeadDev), cudaMemcpyHostToDevice, X),
 	             "upload frame parameters");
 	PHE_CUDA_TRY(cudaEventRecord(r->paramEvents[slot], X), "record parameter slot");
 	for (uint32_t k = 1; k < parts; k++) {   // the other parts' parameters: the same but for part and pixels
 		const uint32_t slotK = r->paramSlot;
 		r->paramSlot = (slotK + 1) % kParamSlots;
 		PHE_CUDA_TRY(cudaEventSynchronize(r->paramEvents[slotK]), "wait for a free parameter slot");
-		FrameParamsDev& fpk = r->hParams[slotK];
+		FrameParamsDev& fpk = r->hParams[slotK].params;
 		fpk = fp;
 		fpk.part = k;
 		fpk.partPixels = n[k];
-		PHE_CUDA_TRY(cudaMemcpyAsync(part_params(r, k), &fpk, sizeof(FrameParamsDev), cudaMemcpyHostToDevice, s),
+		PHE_CUDA_TRY(cudaMemcpyAsync(part_params(r, k), &r->hParams[slotK], sizeof(FrameHeadDev), cudaMemcpyHostToDevice, s),
 		             "upload frame parameters");
 		PHE_CUDA_TRY(cudaEventRecord(r->paramEvents[slotK], s), "record parameter slot");
 	}
@@ -944,7 +951,7 @@ extern "C" phe_status phe_renderer_render(phe_renderer* r, const phe_sphere_ligh
 		if (r->timing) {
 			if ((st = collect_times(r))) return st;
 			r->timedKernels = frame_kernels(r->fused, r->shadowSchedule, r->sortWindow);
-			st = launch_frame(r->scene, r->dParams, r->fb, r->resX, r->resY, s, r->events, r->fused, r->shadowSchedule,
+			st = launch_frame(r->scene, &r->dParams->params, r->fb, r->resX, r->resY, s, r->events, r->fused, r->shadowSchedule,
 			                  nullptr);
 			r->pendingTimes = true;
 		} else {
@@ -1116,4 +1123,4 @@ extern "C" phe_status phe_renderer_read_wait(phe_renderer* r)
 	return PHE_OK;
 }
 
-extern "C" uint32_t phe_renderer_frame_param_bytes(void) { return (uint32_t)sizeof(FrameParamsDev); }
+extern "C" uint32_t phe_renderer_frame_param_bytes(void) { return (uint32_t)sizeof(FrameHeadDev); }

@@ -723,7 +723,6 @@ phe_status launch_frame(const phe_scene* scene, const FrameParamsDev* dParams, c
 	if ((st = device_info(&dinfo))) return st;
 	int binGrid = dinfo->numSMs * 4;
 	if (parts & kFrameTraversal) {
-		PHE_CUDA_TRY(cudaMemsetAsync(fb.counters, 0, sizeof(uint32_t) * kNumCounters, stream), "clear frame counters");
 		mark();
 		if (fused) {
 			const bool wide = scene->dev.nodes4 || scene->dev.nodes8;

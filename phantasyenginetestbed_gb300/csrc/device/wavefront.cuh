@@ -12,7 +12,7 @@ namespace phe_gb300 {
 
 constexpr uint32_t kMaxLights = 8;
 
-// Counters in device memory, cleared at the start of every frame.
+// Counters in device memory, cleared by the upload of every frame's parameters (FrameHeadDev).
 enum : uint32_t {
 	kCtrShadow0 = 0,  // primary shadow-queue length
 	kCtrBounce = 1,   // bounce-queue length
@@ -46,6 +46,14 @@ struct FrameParamsDev {
 	uint32_t part, parts, partPixels, pad;
 };
 
+// What is uploaded before a frame (or a part of one): its parameters and its counters, cleared. One copy instead
+// of a copy and a memset, and a TAA reset with one memset instead of two: a 256x256 frame 140 -> 136 us.
+struct FrameHeadDev {
+	FrameParamsDev params;
+	// a line of their own: in one line with the parameters the counters' atomics made a 1080p frame 6% slower
+	alignas(256) uint32_t counters[kNumCounters];
+};
+
 struct FrameBuffers {
 	float4* contrib;          // [2][L][P] light contributions (primary lights, then bounce lights)
 	uint8_t* inLight;         // [2][L][P] visibility of each contribution
@@ -58,7 +66,7 @@ struct FrameBuffers {
 	float4* rawColor;         // [P] resolved colour before TAA
 	float4* history[2];       // [P] TAA history ping-pong (rgb + effective sample count)
 	float4* color[2];         // [P] TAA output ping-pong (same side as the history it was blended into)
-	uint32_t* counters;       // [kNumCounters]
+	uint32_t* counters;       // [kNumCounters], FrameHeadDev::counters of the frame or part
 	uint32_t capacityLP;      // L * P
 	phe_ray_hit* primaryHits; // [P] closest hits of the primary rays, in 8x8-tile ray order
 	phe_ray_hit* bounceHits;  // [P] closest hits of the bounce queue
@@ -94,7 +102,7 @@ struct FrameStreams {
 	cudaStream_t side = nullptr;
 	cudaEvent_t fork = nullptr, join = nullptr;
 };
-// `parts` selects the traversal kernels (counter reset, primary, bounce, shadow passes), the resolve +
+// `parts` selects the traversal kernels (primary, bounce, shadow passes), the resolve +
 // TAA kernel, or both: a renderer with two frames in flight launches them on different streams.
 enum { kFrameTraversal = 1, kFrameResolve = 2, kFrameAll = 3 };
 // `partPixels` (0 = the whole frame) sizes the grids of one part of a split frame.
