@@ -12,6 +12,7 @@
 // which the autotuner (phe_batch_autotune) picks by timing candidates on the actual batch mix.
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -94,8 +95,12 @@ static phe_status launch_batch_kernel(const BatchTableDev& t, bool wide, int sta
 	auto kernel = wide ? (sh ? batch_kernel<BLOCK, true, kBatchStackShared> : batch_kernel<BLOCK, true, 0>)
 	                   : (sh ? batch_kernel<BLOCK, false, kBatchStackShared> : batch_kernel<BLOCK, false, 0>);
 	const size_t smem = stack_smem_bytes(BLOCK, sh ? kBatchStackShared : 0);
-	int maxB = 0;
-	PHE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxB, kernel, BLOCK, smem), "occupancy");
+	static std::atomic<int> occupancy[2][2] = {};   // [wide][sh]; filled on first use (threads that race store the same value)
+	int maxB = occupancy[wide][sh].load(std::memory_order_relaxed);
+	if (maxB == 0) {
+		PHE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxB, kernel, BLOCK, smem), "occupancy");
+		occupancy[wide][sh].store(maxB, std::memory_order_relaxed);
+	}
 	if (occupancyOut) {
 		*occupancyOut = maxB;
 		return PHE_OK;
