@@ -5,14 +5,6 @@
 
 namespace phe_gb300 {
 
-// getRayIdx (CudaDeviceHelpers.cuh:49-62) for 8x8 tiles when order == 1, row-major otherwise.
-__device__ __forceinline__ uint32_t ray_index(uint32_t x, uint32_t y, uint32_t resX, int order)
-{
-	if (order == 0) return y * resX + x;
-	uint32_t pixBlockIdx = (y >> 3) * (resX >> 3) + (x >> 3);
-	return pixBlockIdx * 64u + (y & 7u) * 8u + (x & 7u);
-}
-
 // calculatePrimaryRayDir (RayCastKernel.cu:891-897) at pixel (x + jx, y + jy):
 // normalize(dir + dX * c.x + dY * c.y), c = loc / res * 2 - 1.
 __device__ __forceinline__ f3 primary_dir(const phe_camera_def& cam, uint32_t x, uint32_t y, uint32_t resX, uint32_t resY,

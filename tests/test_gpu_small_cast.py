@@ -7,7 +7,7 @@ import pytest
 
 import phantasyenginetestbed_gb300 as P
 from oracle import oracle as O
-from tests.helpers import built_scene, device_empty, from_device, random_rays, to_device
+from tests.helpers import C1_CAM, built_scene, cam_struct, device_empty, from_device, random_rays, to_device
 
 pytestmark = pytest.mark.gpu
 N = 400_000   # more than one wave of any device of 152 SMs
@@ -57,3 +57,20 @@ def test_small_launches_give_the_large_launch(name, n):
         assert np.array_equal(vis[:20000], O.any_rays(b.nodes, b.verts, rays[:20000]))
         orc = O.cast_rays(b.nodes, b.verts, rays[:20000], mode=O.MODE_GPU)
         assert O.compare_closest(hits[:20000], orc, rays[:20000], b.slot_to_tri, b.verts)["ok"]
+
+
+@pytest.mark.parametrize("shift", [0, 16])   # the buffer aligned to 32 bytes or to 16 only
+@pytest.mark.parametrize("res,order", [((1, 1), 0), ((257, 3), 0), ((100, 77), 0), ((8, 8), 1), ((264, 24), 1)])
+def test_primary_rays_at_block_edges(res, order, shift):
+    import math
+
+    import torch
+    cam = O.camera_def(C1_CAM["pos"], C1_CAM["dir"], C1_CAM["up"], math.radians(60), res)
+    n = res[0] * res[1]
+    buf = torch.full((shift + n * 32 + 32,), 7, dtype=torch.uint8, device="cuda")
+    P.gen_primary_rays(buf[shift:], cam_struct(cam), res, jitter=(0.25, -0.125), order=order)
+    torch.cuda.synchronize()
+    got = buf.cpu().numpy()
+    want = O.gen_primary(cam, res, jitter=(0.25, -0.125), order=order)
+    assert np.array_equal(got[shift:shift + n * 32], want.view(np.uint8))
+    assert np.all(got[:shift] == 7) and np.all(got[shift + n * 32:] == 7)
