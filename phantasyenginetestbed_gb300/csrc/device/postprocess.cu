@@ -44,15 +44,24 @@ __global__ void postprocess_kernel(uint32_t n, const float4* __restrict__ linear
 // texels never go back. So a warp takes 32 columns and walks kScaleRows rows: a thread keeps the source
 // rows of the current tap, each already filtered along x at both columns, and loads and filters a source
 // row once for all the taps and destination rows that use it, instead of 16 texels a pixel; the rows'
-// positions come from a table that the block computes once. 1920x1080 to 2560x1440: 64 us (56.7 M warp
-// instructions, 16 x 4 one-float loads a pixel) before, 36 without the table. 8 rows a warp: 4 take 2 us longer,
-// 16 the same.
-constexpr int kScaleWarps = 4, kScaleRows = 8;
+// and the columns' positions come from tables that the block computes once, and the filters run on pairs of
+// floats. 1920x1080 to 2560x1440: 64 us (56.7 M warp instructions, 16 x 4 one-float loads a pixel) before, 31 (22.4 M)
+// with scalar filters and the columns computed by every warp, 28 (17.5 M) now. 8 rows a warp: 4 take 2 us longer, 16 the same.
+constexpr int kScaleWarps = 8, kScaleRows = 8;
 constexpr int kScaleTile = kScaleWarps * kScaleRows;   // destination rows of a block
+static_assert(kScaleTile % 32 == 0 && kScaleTile / 32 < kScaleWarps, "a warp is left for the columns' taps");
 
-struct ScaledRow {   // a source row filtered along x at the left and the right column
-	f3 l, r;
+struct ScaledRow {   // a source row filtered along x at the left and the right column: (x, y) of each, both z
+	f32x2 l, r, z;
 };
+// glsl_mix of both lanes, with the weights (w1, w1) = 1 - t and (w2, w2) = t.
+__device__ __forceinline__ f32x2 mix2(f32x2 a, f32x2 b, f32x2 w1, f32x2 w2)
+{
+	float a0, a1, b0, b1;
+	unpack2(mul2(a, w1), a0, a1);
+	unpack2(mul2(b, w2), b0, b1);
+	return pack2(__fadd_rn(a0, b0), __fadd_rn(a1, b1));
+}
 template <bool VEC>
 __device__ __forceinline__ ScaledRow scaled_row(const float4* __restrict__ src, uint32_t W, uint32_t row, const LinearAxis& xl,
                                                 const LinearAxis& xr)
@@ -60,36 +69,39 @@ __device__ __forceinline__ ScaledRow scaled_row(const float4* __restrict__ src, 
 	const float4* p = src + (size_t)row * W;
 	const float4 a = ld_texel<VEC>(p + xl.i0), b = ld_texel<VEC>(p + xl.i1);
 	const float4 c = ld_texel<VEC>(p + xr.i0), d = ld_texel<VEC>(p + xr.i1);
+	const float wl = __fsub_rn(1.0f, xl.a), wr = __fsub_rn(1.0f, xr.a);
 	ScaledRow o;
-	o.l = mk3(glsl_mix(a.x, b.x, xl.a), glsl_mix(a.y, b.y, xl.a), glsl_mix(a.z, b.z, xl.a));
-	o.r = mk3(glsl_mix(c.x, d.x, xr.a), glsl_mix(c.y, d.y, xr.a), glsl_mix(c.z, d.z, xr.a));
+	o.l = mix2(pack2(a.x, a.y), pack2(b.x, b.y), pack2(wl, wl), pack2(xl.a, xl.a));
+	o.r = mix2(pack2(c.x, c.y), pack2(d.x, d.y), pack2(wr, wr), pack2(xr.a, xr.a));
+	o.z = pack2(glsl_mix(a.z, b.z, xl.a), glsl_mix(c.z, d.z, xr.a));
 	return o;
 }
-__device__ __forceinline__ f3 mix3(f3 a, f3 b, float t) { return mk3(glsl_mix(a.x, b.x, t), glsl_mix(a.y, b.y, t), glsl_mix(a.z, b.z, t)); }
 
 template <bool VEC>
 __global__ void __launch_bounds__(32 * kScaleWarps)
 scale_kernel(uint32_t srcW, uint32_t srcH, const float4* __restrict__ src, float vpW, float vpH, uint32_t dstW, uint32_t dstH,
              float4* __restrict__ dst, uchar4* __restrict__ rgba8)
 {
-	__shared__ LinearAxis rowTop[kScaleTile], rowBottom[kScaleTile];   // the taps of the block's rows
+	// the taps of the block's rows and columns, each computed once
+	__shared__ LinearAxis rowTop[kScaleTile], rowBottom[kScaleTile], colLeft[32], colRight[32];
 	const uint32_t x = blockIdx.x * 32u + threadIdx.x;
 	const uint32_t yBlock = blockIdx.y * kScaleTile, yFirst = yBlock + threadIdx.y * kScaleRows;
 	const uint32_t yEnd = min(dstH, yFirst + kScaleRows);
-	const float dw = (float)dstW, dh = (float)dstH, sw = (float)srcW, sh = (float)srcH;
-	const float ox = __fmul_rn(__fdiv_rn(1.0f, dw), 0.25f), oy = __fmul_rn(__fdiv_rn(1.0f, dh), 0.25f);
-	const uint32_t row = threadIdx.y * 32u + threadIdx.x;
-	if (row < kScaleTile) {
-		const float cy = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)(yBlock + row), 0.5f), dh), vpH), sh);
-		rowTop[row] = linear_axis(__fmul_rn(__fadd_rn(cy, -oy), sh), srcH);
-		rowBottom[row] = linear_axis(__fmul_rn(__fadd_rn(cy, oy), sh), srcH);
+	const uint32_t t = threadIdx.y * 32u + threadIdx.x;
+	if (t < kScaleTile) {
+		const float dh = (float)dstH, sh = (float)srcH, oy = __fmul_rn(__fdiv_rn(1.0f, dh), 0.25f);
+		const float cy = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)(yBlock + t), 0.5f), dh), vpH), sh);
+		rowTop[t] = linear_axis(__fmul_rn(__fadd_rn(cy, -oy), sh), srcH);
+		rowBottom[t] = linear_axis(__fmul_rn(__fadd_rn(cy, oy), sh), srcH);
+	} else if (threadIdx.y == kScaleTile / 32) {
+		// columns beyond the last repeat it, so that the warps stay whole; their lanes store nothing
+		const float dw = (float)dstW, sw = (float)srcW, ox = __fmul_rn(__fdiv_rn(1.0f, dw), 0.25f);
+		const float cx = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)min(x, dstW - 1), 0.5f), dw), vpW), sw);
+		colLeft[threadIdx.x] = linear_axis(__fmul_rn(__fadd_rn(cx, -ox), sw), srcW);
+		colRight[threadIdx.x] = linear_axis(__fmul_rn(__fadd_rn(cx, ox), sw), srcW);
 	}
 	__syncthreads();
-	// lanes beyond the last column repeat it, so that the warp stays whole; they store nothing
-	const uint32_t xc = min(x, dstW - 1);
-	const float cx = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)xc, 0.5f), dw), vpW), sw);
-	const LinearAxis xl = linear_axis(__fmul_rn(__fadd_rn(cx, -ox), sw), srcW);
-	const LinearAxis xr = linear_axis(__fmul_rn(__fadd_rn(cx, ox), sw), srcW);
+	const LinearAxis xl = colLeft[threadIdx.x], xr = colRight[threadIdx.x];
 	// source rows held in r0 and r1 (none yet)
 	uint32_t have0 = 0xFFFFFFFFu, have1 = 0xFFFFFFFFu;
 	ScaledRow r0{}, r1{};
@@ -105,12 +117,21 @@ scale_kernel(uint32_t srcW, uint32_t srcH, const float4* __restrict__ src, float
 	};
 	for (uint32_t y = yFirst; y < yEnd; y++) {
 		const LinearAxis yt = rowTop[y - yBlock], yb = rowBottom[y - yBlock];
+		f3 acc;
+		auto tap = [&](float t, bool first) {
+			const float u = __fsub_rn(1.0f, t);
+			const f32x2 w1 = pack2(u, u), w2 = pack2(t, t);
+			float lx, ly, rx, ry, lz, rz;
+			unpack2(mix2(r0.l, r1.l, w1, w2), lx, ly);
+			unpack2(mix2(r0.r, r1.r, w1, w2), rx, ry);
+			unpack2(mix2(r0.z, r1.z, w1, w2), lz, rz);
+			const f3 l = mk3(lx, ly, lz);
+			acc = add3(first ? l : add3(acc, l), mk3(rx, ry, rz));
+		};
 		need(yt.i0, yt.i1);
-		f3 acc = mix3(r0.l, r1.l, yt.a);
-		acc = add3(acc, mix3(r0.r, r1.r, yt.a));
+		tap(yt.a, true);
 		need(yb.i0, yb.i1);
-		acc = add3(acc, mix3(r0.l, r1.l, yb.a));
-		acc = add3(acc, mix3(r0.r, r1.r, yb.a));
+		tap(yb.a, false);
 		const float4 o = make_float4(__fmul_rn(acc.x, 0.25f), __fmul_rn(acc.y, 0.25f), __fmul_rn(acc.z, 0.25f), 1.0f);
 		if (x >= dstW) continue;
 		const size_t p = (size_t)y * dstW + x;
