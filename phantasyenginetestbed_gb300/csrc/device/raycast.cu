@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(kPlainBlock, kCastMinBlocks) closest_plain_ker
 __device__ __forceinline__ uint32_t next_rays(uint32_t* __restrict__ counter)
 {
 	if (!counter) return 0xFFFFFFFFu;
+	wait_for_previous();   // the counter is cleared
 	uint32_t base = 0;
 	if ((threadIdx.x & 31u) == 0) base = gridDim.x * blockDim.x + atomicAdd(counter, 32u);
 	return __shfl_sync(0xffffffffu, base, 0);
@@ -259,12 +260,11 @@ extern "C" phe_status phe_cast_closest(const phe_scene* scene, const phe_ray_in*
 	if ((st = persistent_grid(wide ? 2 : 0, (const void*)kernel, &grid))) return st;
 	uint32_t maxGrid = (n + kPersistentBlock - 1) / kPersistentBlock;
 	uint32_t* counter = nullptr;
+	bool early = false;
 	if ((uint32_t)grid >= maxGrid) grid = (int)maxGrid;   // one wave: no counter
-	else if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
-	kernel<<<grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream>>>(scene->dev, rays, hits,
-	                                                                                             n, counter,
-	                                                                                             scene->status);
-	PHE_CUDA_TRY(cudaGetLastError(), "closest_persistent_kernel launch");
+	else if ((st = acquire_counter((cudaStream_t)stream, &counter, &early))) return st;
+	PHE_CUDA_TRY(launch_early(early, kernel, grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream,
+	                          scene->dev, rays, hits, n, counter, scene->status), "closest_persistent_kernel launch");
 	return PHE_OK;
 }
 
@@ -283,12 +283,10 @@ extern "C" phe_status phe_cast_any(const phe_scene* scene, const phe_ray_in* ray
 	if ((st = persistent_grid(wide ? 3 : 1, (const void*)kernel, &grid))) return st;
 	uint32_t maxGrid = (n + kPersistentBlock - 1) / kPersistentBlock;
 	uint32_t* counter = nullptr;
+	bool early = false;
 	if ((uint32_t)grid >= maxGrid) grid = (int)maxGrid;   // one wave: no counter
-	else if ((st = acquire_counter((cudaStream_t)stream, &counter))) return st;
-	kernel<<<grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream>>>(scene->dev, rays,
-	                                                                                             inLight, scatter, n,
-	                                                                                             counter,
-	                                                        scene->status);
-	PHE_CUDA_TRY(cudaGetLastError(), "any_persistent_kernel launch");
+	else if ((st = acquire_counter((cudaStream_t)stream, &counter, &early))) return st;
+	PHE_CUDA_TRY(launch_early(early, kernel, grid, kPersistentBlock, stack_smem_bytes(kPersistentBlock), (cudaStream_t)stream,
+	                          scene->dev, rays, inLight, scatter, n, counter, scene->status), "any_persistent_kernel launch");
 	return PHE_OK;
 }

@@ -40,8 +40,42 @@ constexpr uint32_t kMaxPersistentRays = PHE_MAX_PERSISTENT_RAYS;
 
 // Returns the runtime state of the current device, initialising it on first use.
 phe_status device_info(DeviceInfo** out);
-// A zeroed work counter for one persistent launch on `stream` (a memset is queued on the stream).
-phe_status acquire_counter(cudaStream_t stream, uint32_t** counter);
+// A zeroed work counter for one persistent launch on `stream`. It is cleared by work queued on the stream: a memset
+// in a stream that is being captured (*early false), else a kernel that lets the next one start beside it (*early
+// true): launch_early the persistent kernel, which waits (wait_for_previous) before it first uses the counter.
+phe_status acquire_counter(cudaStream_t stream, uint32_t** counter, bool* early);
+
+// Programmatic launches: a kernel queued with launch_early starts as soon as every block of the kernel before it on
+// the stream has left or has said let_next_start, so its launch is not waited for; what that kernel wrote may be read
+// after wait_for_previous (a no-op in a kernel launched otherwise). The kernel before it never waits for this one.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Whether launches on `stream` go into a graph (or may not be made now: the launch itself then reports why).
+inline bool stream_captures(cudaStream_t stream)
+{
+	cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(stream, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+	cudaGetLastError();
+	return true;
+}
+
+template <class... P, class... A>
+cudaError_t launch_early(bool early, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream, A... args)
+{
+	cudaLaunchAttribute at = {};
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t c = {};
+	c.gridDim = dim3(grid);
+	c.blockDim = dim3(block);
+	c.dynamicSmemBytes = smem;
+	c.stream = stream;
+	c.attrs = &at;
+	c.numAttrs = early ? 1 : 0;
+	cudaLaunchKernelEx(&c, kernel, P(args)...);
+	return cudaGetLastError();
+}
 
 inline phe_status cuda_fail(cudaError_t e, const char* what)
 {

@@ -45,14 +45,28 @@ phe_status device_info(DeviceInfo** out)
 	return PHE_OK;
 }
 
-phe_status acquire_counter(cudaStream_t stream, uint32_t** counter)
+// 200,000 shadow rays on 10K triangles take 22.9 us after a memset, 22.4 us with this; 778K on 155K 92.4 -> 91.9 us,
+// 1M diffuse rays 293.5 -> 292.6 us: the cast kernel is on the chip, at its first rays, when the counter is cleared.
+__global__ void clear_counter_kernel(uint32_t* counter)
+{
+	let_next_start();
+	*counter = 0;
+}
+
+phe_status acquire_counter(cudaStream_t stream, uint32_t** counter, bool* early)
 {
 	DeviceInfo* d = nullptr;
 	phe_status s = device_info(&d);
 	if (s) return s;
 	uint32_t slot = g_counterNext.fetch_add(1) % kCounterPool;
 	uint32_t* c = d->counterPool + slot;
-	PHE_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(uint32_t), stream), "cudaMemsetAsync(counter)");
+	*early = !stream_captures(stream);
+	if (*early) {
+		clear_counter_kernel<<<1, 1, 0, stream>>>(c);
+		PHE_CUDA_TRY(cudaGetLastError(), "clear_counter_kernel launch");
+	} else {
+		PHE_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(uint32_t), stream), "cudaMemsetAsync(counter)");
+	}
 	*counter = c;
 	return PHE_OK;
 }

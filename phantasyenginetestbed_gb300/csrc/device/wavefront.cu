@@ -215,13 +215,14 @@ __global__ void __launch_bounds__(kWaveBlock, kWaveMinBlocks) primary_kernel(Dev
 template <bool WIDE>
 __global__ void __launch_bounds__(kWaveBlock) any_queue_kernel(DeviceScene s, const phe_ray_in* __restrict__ raysA,
                                                                const uint32_t* __restrict__ slotsA,
-                                                               const uint32_t* __restrict__ countA,
+                                                               const uint32_t* countA,
                                                                const phe_ray_in* __restrict__ raysB,
                                                                const uint32_t* __restrict__ slotsB,
-                                                               const uint32_t* __restrict__ countB,
+                                                               const uint32_t* countB,
                                                                uint8_t* __restrict__ inLight, uint32_t* __restrict__ work,
                                                                uint32_t* __restrict__ status)
 {
+	wait_for_previous();
 	const uint32_t nA = *countA, n = nA + (countB ? *countB : 0u);
 	uint32_t base = first_work();
 	while (base < n) {
@@ -273,6 +274,7 @@ template <bool WIDE>
 __global__ void __launch_bounds__(kWaveBlock, kBounceMinBlocks) bounce_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
                                                             FrameBuffers fb, uint32_t* __restrict__ status)
 {
+	wait_for_previous();
 	const FrameParamsDev& fp = *fpp;
 	const uint32_t P = fp.numPixels, L = fp.numLights;
 	const uint32_t n = fb.counters[kCtrBounce];
@@ -556,6 +558,7 @@ constexpr uint32_t kResolveChunk = 2;   // light slots whose loads are issued to
 __global__ void __launch_bounds__(kResolveBlock, kResolveMinBlocks)
 resolve_taa_kernel(const FrameParamsDev* __restrict__ fpp, FrameBuffers fb)
 {
+	wait_for_previous();
 	const FrameParamsDev& fp = *fpp;
 	const uint32_t P = fp.numPixels, L = fp.numLights, np = fp.partPixels, W = fp.resX;
 	// The thread's two pixels, indices q0 and q1 into this part's pixels in row order (the part's rows
@@ -728,6 +731,10 @@ phe_status launch_frame(const phe_scene* scene, const FrameParamsDev* dParams, c
 	DeviceInfo* dinfo = nullptr;
 	if ((st = device_info(&dinfo))) return st;
 	int binGrid = dinfo->numSMs * 4;
+	// A stage is queued to start while the one before it ends (launch_early), unless an event is recorded between the
+	// two or the frame goes into a graph, whose own edges measured the same: a 256x256 frame on 10K triangles 129 ->
+	// 121 us, two 256x144 frames in flight 98 -> 94.5 us each on 155K, 0.5-1% at 1080p.
+	const bool early = !ev && !stream_captures(stream);
 	if (parts & kFrameTraversal) {
 		mark();
 		if (fused) {
@@ -765,13 +772,14 @@ phe_status launch_frame(const phe_scene* scene, const FrameParamsDev* dParams, c
 				bin_bounce_kernel<<<binGrid, kBinBlock, 0, stream>>>(fb);
 				mark();
 			}
-			bounce<<<gBounce, kWaveBlock, kStackSmem, stream>>>(scene->dev, dParams, fb, scene->status);
+			PHE_CUDA_TRY(launch_early(early, bounce, gBounce, kWaveBlock, kStackSmem, stream, scene->dev, dParams, fb, scene->status),
+			             "bounce_kernel launch");
 			mark();
 			if (schedule == PHE_SHADOWS_MERGED) {
 				// bounce shadows first: their incoherent rays start early and the primary ones fill the tail
-				anyQueue<<<gAny, kWaveBlock, kStackSmem, stream>>>(scene->dev, rays1, slots1, fb.counters + kCtrShadow1,
-				                                           fb.shadowRays, fb.shadowSlots, fb.counters + kCtrShadow0,
-				                                           fb.inLight, fb.counters + kCtrWork3, scene->status);
+				PHE_CUDA_TRY(launch_early(early, anyQueue, gAny, kWaveBlock, kStackSmem, stream, scene->dev, rays1, slots1,
+				                          fb.counters + kCtrShadow1, fb.shadowRays, fb.shadowSlots, fb.counters + kCtrShadow0,
+				                          fb.inLight, fb.counters + kCtrWork3, scene->status), "any_queue_kernel launch");
 			} else {
 				anyQueue<<<gAny, kWaveBlock, kStackSmem, stream>>>(scene->dev, rays1, slots1, fb.counters + kCtrShadow1, nullptr,
 				                                           nullptr, nullptr, fb.inLight, fb.counters + kCtrWork3,
@@ -808,7 +816,8 @@ phe_status launch_frame(const phe_scene* scene, const FrameParamsDev* dParams, c
 	if (parts & kFrameResolve) {
 		const uint64_t pixels = partPixels ? partPixels : (uint64_t)resX * resY;
 		const uint32_t resolveGrid = (uint32_t)((pixels + 2 * kResolveBlock - 1) / (2 * kResolveBlock));
-		resolve_taa_kernel<<<resolveGrid, kResolveBlock, 0, stream>>>(dParams, fb);
+		PHE_CUDA_TRY(launch_early(early && (parts & kFrameTraversal), resolve_taa_kernel, resolveGrid, kResolveBlock, 0, stream,
+		                          dParams, fb), "resolve_taa_kernel launch");
 		mark();
 	}
 	PHE_CUDA_TRY(cudaGetLastError(), "frame kernel launch");

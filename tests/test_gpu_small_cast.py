@@ -74,3 +74,44 @@ def test_primary_rays_at_block_edges(res, order, shift):
     want = O.gen_primary(cam, res, jitter=(0.25, -0.125), order=order)
     assert np.array_equal(got[shift:shift + n * 32], want.view(np.uint8))
     assert np.all(got[:shift] == 7) and np.all(got[shift + n * 32:] == 7)
+
+
+@pytest.mark.parametrize("n", [152 * 1280 + 1, 300_001])
+def test_counter_cleared_in_and_out_of_a_graph(n):
+    """Rays written by the work before on the stream; cleared by a kernel that runs beside the cast, or by a memset
+    inside a graph, replayed."""
+    import torch
+    _, scene, _, d_rays, hits, vis = _large("c2_256_2000")
+    stream = torch.cuda.Stream()
+    rays, out = torch.empty_like(d_rays), device_empty(n, P.RAY_HIT_DTYPE)
+    lit = device_empty(n, np.uint8)
+
+    def work():
+        rays.copy_(d_rays)
+        P.cast_closest(scene, rays, out, n, stream=stream)
+        rays.zero_()
+        rays.copy_(d_rays)
+        P.cast_any(scene, rays, lit, n, stream=stream)
+        rays.zero_()
+
+    def check():
+        stream.synchronize()
+        assert np.array_equal(from_device(out, np.uint8), hits[:n].view(np.uint8))
+        assert np.array_equal(from_device(lit, np.uint8), vis[:n])
+        assert scene.status() == 0
+        out.zero_()
+        lit.zero_()
+        torch.cuda.synchronize()
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            work()
+        check()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        work()
+    for _ in range(2):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        check()
