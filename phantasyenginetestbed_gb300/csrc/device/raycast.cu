@@ -21,9 +21,10 @@ constexpr int kPersistentBlock = 128;
 // 10 resident blocks of 128 per SM (48 registers): 9 (the compiler's 52 registers) and 8 made 1M diffuse rays
 // 1% and 4% slower, 12 (40 registers, spills) 12%.
 constexpr int kCastMinBlocks = 10;
+constexpr int cast_min_blocks(bool wide) { return wide ? kWideMinBlocks : kCastMinBlocks; }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kPlainBlock, kCastMinBlocks) closest_plain_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays,
+__global__ void __launch_bounds__(kPlainBlock, cast_min_blocks(WIDE)) closest_plain_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays,
                                                                     phe_ray_hit* __restrict__ hits, uint32_t n,
                                                                     uint32_t* __restrict__ status)
 {
@@ -51,7 +52,7 @@ __device__ __forceinline__ uint32_t next_rays(uint32_t* __restrict__ counter)
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) closest_persistent_kernel(DeviceScene s,
+__global__ void __launch_bounds__(kPersistentBlock, cast_min_blocks(WIDE)) closest_persistent_kernel(DeviceScene s,
                                                                               const phe_ray_in* __restrict__ rays,
                                                                               phe_ray_hit* __restrict__ hits, uint32_t n,
                                                                               uint32_t* __restrict__ counter,
@@ -135,7 +136,7 @@ small_cast_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays, void* __re
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kPersistentBlock, kCastMinBlocks) any_persistent_kernel(DeviceScene s,
+__global__ void __launch_bounds__(kPersistentBlock, cast_min_blocks(WIDE)) any_persistent_kernel(DeviceScene s,
                                                                           const phe_ray_in* __restrict__ rays,
                                                                           uint8_t* __restrict__ inLight,
                                                                           const uint32_t* __restrict__ scatter, uint32_t n,

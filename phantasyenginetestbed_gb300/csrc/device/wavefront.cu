@@ -137,7 +137,7 @@ __device__ __forceinline__ uint32_t next_work(uint32_t* __restrict__ work)
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kWaveBlock, kWaveMinBlocks) primary_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
+__global__ void __launch_bounds__(kWaveBlock, WIDE ? kWideMinBlocks : kWaveMinBlocks) primary_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
                                                              FrameBuffers fb, uint32_t* __restrict__ status)
 {
 	const FrameParamsDev& fp = *fpp;
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kBinBlock) bin_bounce_kernel(FrameBuffers fb)
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kWaveBlock, kBounceMinBlocks) bounce_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
+__global__ void __launch_bounds__(kWaveBlock, WIDE ? kWideMinBlocks : kBounceMinBlocks) bounce_kernel(DeviceScene s, const FrameParamsDev* __restrict__ fpp,
                                                             FrameBuffers fb, uint32_t* __restrict__ status)
 {
 	wait_for_previous();
