@@ -59,3 +59,33 @@ def test_taa_edges(res, shift):
     want_c, want_h = O.taa(cur, hist, rough, vel, pvel)
     assert np.array_equal(from_device(oc, np.float32).reshape(H, W, 4), want_c)
     assert np.array_equal(from_device(oh, np.float32).reshape(H, W, 4), want_h)
+
+
+@pytest.mark.parametrize("rows", [6079, 6080, 12160, 24319, 24323])   # 1, 2, 4, 4 and 8 rows a warp on 152 SMs
+def test_scaling_rows_per_warp(rows):
+    import torch
+    img = np.random.default_rng(rows).uniform(0, 1.2, (29, 37, 4)).astype(np.float32)
+    d_dst = device_empty(31 * rows, np.dtype((np.float32, 4)))
+    scale((37, 29), to_device(img), (31, rows), d_dst)
+    torch.cuda.synchronize()
+    assert np.array_equal(from_device(d_dst, np.float32).reshape(rows, 31, 4), O.scale(img, (31, rows)))
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("res", [(1, 1), (33, 5), (64, 4)])
+def test_taa_without_velocities(res, shift):
+    import torch
+    W, H = res
+    rng = np.random.default_rng(W * H)
+    cur, hist = (rng.uniform(0, 2, (H, W, 4)).astype(np.float32) for _ in range(2))
+    pvel = (rng.normal(size=(H, W, 2)) * 0.05).astype(np.float32)
+    rough = rng.uniform(0, 1, (H, W)).astype(np.float32)
+    for prev in (None, pvel):
+        oc, oh = (device_empty(W * H, np.dtype((np.float32, 4))) for _ in range(2))
+        taa_resolve(res, to_device(cur), _floats(hist, shift), oc, oh, None, None if prev is None else _floats(prev, shift),
+                    to_device(rough))
+        torch.cuda.synchronize()
+        zero = np.zeros((H, W, 2), np.float32)
+        want_c, want_h = O.taa(cur, hist, rough, zero, zero if prev is None else prev)
+        assert np.array_equal(from_device(oc, np.float32).reshape(H, W, 4), want_c)
+        assert np.array_equal(from_device(oh, np.float32).reshape(H, W, 4), want_h)
