@@ -41,15 +41,17 @@ __global__ void postprocess_kernel(uint32_t n, const float4* __restrict__ linear
 // four GL_LINEAR taps at +-1/4 destination pixel, averaged; alpha 1.
 //
 // The four taps are two columns by two rows of positions, and down a destination column the rows' source
-// texels never go back. So a warp takes 32 columns and walks kScaleRows rows: a thread keeps the source
+// texels never go back. So a warp takes 32 columns and walks ROWS rows: a thread keeps the source
 // rows of the current tap, each already filtered along x at both columns, and loads and filters a source
 // row once for all the taps and destination rows that use it, instead of 16 texels a pixel; the rows'
 // and the columns' positions come from tables that the block computes once, and the filters run on pairs of
 // floats. 1920x1080 to 2560x1440: 64 us (56.7 M warp instructions, 16 x 4 one-float loads a pixel) before, 31 (22.4 M)
-// with scalar filters and the columns computed by every warp, 28 (17.5 M) now. 8 rows a warp: 4 take 2 us longer, 16 the same.
-constexpr int kScaleWarps = 8, kScaleRows = 8;
-constexpr int kScaleTile = kScaleWarps * kScaleRows;   // destination rows of a block
-static_assert(kScaleTile % 32 == 0 && kScaleTile / 32 < kScaleWarps, "a warp is left for the columns' taps");
+// with scalar filters and the columns computed by every warp, 28 (17.5 M) now, with 8 rows a warp (4: 2 us longer, 16: the same).
+//
+// A small image has too few warps at 8 rows each: a warp takes 1, 2, 4 or 8 rows, as many as leave 20 warps an SM.
+// Tonemap and scaling of 640x360 to 300x200 / 640x360 / 901x503 / 1280x720 at 1, 2, 4 and 8 rows: 10.4 12.4 13.3 16.5 /
+// 12.5 12.4 12.4 14.5 / 14.5 13.6 12.4 14.5 / 18.6 16.5 14.5 14.8 us (12.4 / 15.5 / 18.6 / 28.8 with 16 loads a pixel).
+constexpr int kScaleWarps = 8, kScaleWarpsPerSM = 20;
 
 struct ScaledRow {   // a source row filtered along x at the left and the right column: (x, y) of each, both z
 	f32x2 l, r, z;
@@ -77,23 +79,25 @@ __device__ __forceinline__ ScaledRow scaled_row(const float4* __restrict__ src, 
 	return o;
 }
 
-template <bool VEC>
+template <bool VEC, int ROWS>
 __global__ void __launch_bounds__(32 * kScaleWarps)
 scale_kernel(uint32_t srcW, uint32_t srcH, const float4* __restrict__ src, float vpW, float vpH, uint32_t dstW, uint32_t dstH,
              float4* __restrict__ dst, uchar4* __restrict__ rgba8)
 {
+	constexpr int kTile = ROWS * kScaleWarps;   // rows of a block
+	static_assert(kTile <= 32 * (kScaleWarps - 1), "the last warp fills the columns' table");
 	// the taps of the block's rows and columns, each computed once
-	__shared__ LinearAxis rowTop[kScaleTile], rowBottom[kScaleTile], colLeft[32], colRight[32];
+	__shared__ LinearAxis rowTop[kTile], rowBottom[kTile], colLeft[32], colRight[32];
 	const uint32_t x = blockIdx.x * 32u + threadIdx.x;
-	const uint32_t yBlock = blockIdx.y * kScaleTile, yFirst = yBlock + threadIdx.y * kScaleRows;
-	const uint32_t yEnd = min(dstH, yFirst + kScaleRows);
+	const uint32_t yBlock = blockIdx.y * kTile, yFirst = yBlock + threadIdx.y * ROWS;
+	const uint32_t yEnd = min(dstH, yFirst + ROWS);
 	const uint32_t t = threadIdx.y * 32u + threadIdx.x;
-	if (t < kScaleTile) {
+	if (t < kTile) {
 		const float dh = (float)dstH, sh = (float)srcH, oy = __fmul_rn(__fdiv_rn(1.0f, dh), 0.25f);
 		const float cy = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)(yBlock + t), 0.5f), dh), vpH), sh);
 		rowTop[t] = linear_axis(__fmul_rn(__fadd_rn(cy, -oy), sh), srcH);
 		rowBottom[t] = linear_axis(__fmul_rn(__fadd_rn(cy, oy), sh), srcH);
-	} else if (threadIdx.y == kScaleTile / 32) {
+	} else if (threadIdx.y == kScaleWarps - 1) {
 		// columns beyond the last repeat it, so that the warps stay whole; their lanes store nothing
 		const float dw = (float)dstW, sw = (float)srcW, ox = __fmul_rn(__fdiv_rn(1.0f, dw), 0.25f);
 		const float cx = __fdiv_rn(__fmul_rn(__fdiv_rn(__fadd_rn((float)min(x, dstW - 1), 0.5f), dw), vpW), sw);
@@ -153,11 +157,21 @@ extern "C" phe_status phe_scale(uint32_t srcW, uint32_t srcH, const float* src, 
 	if (srcW > 65536 || srcH > 65536 || dstW > 65536 || dstH > 65536)
 		return fail(PHE_ERR_TOO_LARGE, "phe_scale: images are limited to 65536 x 65536");
 	if (!dstW || !dstH) return PHE_OK;
-	dim3 block(32, kScaleWarps);
-	dim3 grid((dstW + 31) / 32, (dstH + kScaleTile - 1) / kScaleTile);
-	auto kernel = ((uintptr_t)src & 15u) ? scale_kernel<false> : scale_kernel<true>;   // src may be aligned to floats only
-	kernel<<<grid, block, 0, (cudaStream_t)stream>>>(srcW, srcH, (const float4*)src, (float)viewportW, (float)viewportH, dstW,
-	                                                 dstH, (float4*)dst, (uchar4*)dstRgba8);
+	int dev = 0, numSMs = 0;
+	PHE_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+	PHE_CUDA_TRY(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, dev), "SM count");
+	// rows of a warp: as many as leave kScaleWarpsPerSM warps an SM
+	const uint64_t strips = (uint64_t)((dstW + 31) / 32) * dstH;   // rows of 32 columns
+	int k = 0;
+	while (k < 3 && strips >> (k + 1) >= (uint64_t)kScaleWarpsPerSM * (uint32_t)numSMs) k++;
+	const bool vec = !((uintptr_t)src & 15u);   // src may be aligned to floats only
+	using Kernel = decltype(&scale_kernel<true, 1>);
+	static constexpr Kernel kernels[2][4] = {
+		{scale_kernel<false, 1>, scale_kernel<false, 2>, scale_kernel<false, 4>, scale_kernel<false, 8>},
+		{scale_kernel<true, 1>, scale_kernel<true, 2>, scale_kernel<true, 4>, scale_kernel<true, 8>}};
+	const uint32_t tile = (uint32_t)kScaleWarps << k;
+	kernels[vec][k]<<<dim3((dstW + 31) / 32, (dstH + tile - 1) / tile), dim3(32, kScaleWarps), 0, (cudaStream_t)stream>>>(
+		srcW, srcH, (const float4*)src, (float)viewportW, (float)viewportH, dstW, dstH, (float4*)dst, (uchar4*)dstRgba8);
 	PHE_CUDA_TRY(cudaGetLastError(), "scale_kernel launch");
 	return PHE_OK;
 }
