@@ -58,8 +58,11 @@ template <int BLOCK, bool WIDE, int SN>
 __global__ void __launch_bounds__(BLOCK, kBatchThreadsPerSM / BLOCK) batch_kernel(BatchTableDev t, uint32_t* __restrict__ counter)
 {
 	const uint32_t lane = threadIdx.x & 31u;
-	uint32_t g = (blockIdx.x * BLOCK + threadIdx.x) & ~31u;
-	while (g < t.totalPadded) {
+	for (;;) {
+		uint32_t g = 0;
+		if (lane == 0) g = atomicAdd(counter, 32u);
+		g = __shfl_sync(0xFFFFFFFFu, g, 0);
+		if (g >= t.totalPadded) break;
 		uint32_t it = find_item(t.items, t.numItems, g);
 		const BatchItemDev item = t.items[it];
 		uint32_t i = g - item.base + lane;
@@ -79,10 +82,6 @@ __global__ void __launch_bounds__(BLOCK, kBatchThreadsPerSM / BLOCK) batch_kerne
 			if (err) atomicOr(s.status, err);
 		}
 		__syncwarp();
-		if (!counter) break;
-		wait_for_previous();
-		if (lane == 0) g = gridDim.x * BLOCK + atomicAdd(counter, 32u);
-		g = __shfl_sync(0xFFFFFFFFu, g, 0);
 	}
 }
 
@@ -110,14 +109,9 @@ static phe_status launch_batch_kernel(const BatchTableDev& t, bool wide, int sta
 	if (b < 1) b = 1;
 	uint32_t grid = (uint32_t)(b * numSMs);
 	uint32_t need = (t.totalPadded + BLOCK - 1) / BLOCK;
-	bool early = false;
-	if (grid >= need) {   // one wave: no counter
-		grid = need > 0 ? need : 1;
-		counter = nullptr;
-	} else if (phe_status st = clear_counter(stream, counter, &early)) {
-		return st;
-	}
-	PHE_CUDA_TRY(launch_early(early, kernel, grid, BLOCK, smem, stream, t, counter), "batch_kernel launch");
+	if (grid > need) grid = need > 0 ? need : 1;
+	kernel<<<grid, BLOCK, smem, stream>>>(t, counter);
+	PHE_CUDA_TRY(cudaGetLastError(), "batch_kernel launch");
 	return PHE_OK;
 }
 
@@ -400,6 +394,7 @@ static phe_status batch_enqueue(phe_batch* b, cudaStream_t stream)
 	if (st) return st;
 	const bool sorted = b->params.sortWindow > 0 && b->numWindows > 0;
 	BatchTableDev t{b->dItems, b->dScenes, (uint32_t)b->items.size(), b->totalPadded, sorted ? b->dPerm : nullptr};
+	PHE_CUDA_TRY(cudaMemsetAsync(b->dCounter, 0, sizeof(uint32_t), stream), "clear batch counter");
 	if (b->totalPadded == 0) return PHE_OK;
 	if (sorted) {
 		uint32_t grid = std::min<uint32_t>(b->numWindows, (uint32_t)d->numSMs * 8u);

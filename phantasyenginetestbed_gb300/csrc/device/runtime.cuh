@@ -40,11 +40,9 @@ constexpr uint32_t kMaxPersistentRays = PHE_MAX_PERSISTENT_RAYS;
 
 // Returns the runtime state of the current device, initialising it on first use.
 phe_status device_info(DeviceInfo** out);
-// Clears a work counter for the persistent launch queued next on `stream`: a memset in a stream that is being captured
-// (*early false), else a kernel that lets the next one start beside it (*early true): launch_early the persistent
-// kernel, which waits (wait_for_previous) before it first uses the counter.
-phe_status clear_counter(cudaStream_t stream, uint32_t* counter, bool* early);
-// A work counter of the device's pool, cleared so.
+// A zeroed work counter for one persistent launch on `stream`. It is cleared by work queued on the stream: a memset
+// in a stream that is being captured (*early false), else a kernel that lets the next one start beside it (*early
+// true): launch_early the persistent kernel, which waits (wait_for_previous) before it first uses the counter.
 phe_status acquire_counter(cudaStream_t stream, uint32_t** counter, bool* early);
 
 // Programmatic launches: a kernel queued with launch_early starts as soon as every block of the kernel before it on

@@ -53,25 +53,22 @@ __global__ void clear_counter_kernel(uint32_t* counter)
 	*counter = 0;
 }
 
-phe_status clear_counter(cudaStream_t stream, uint32_t* counter, bool* early)
-{
-	*early = !stream_captures(stream);
-	if (*early) {
-		clear_counter_kernel<<<1, 1, 0, stream>>>(counter);
-		PHE_CUDA_TRY(cudaGetLastError(), "clear_counter_kernel launch");
-	} else {
-		PHE_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream), "cudaMemsetAsync(counter)");
-	}
-	return PHE_OK;
-}
-
 phe_status acquire_counter(cudaStream_t stream, uint32_t** counter, bool* early)
 {
 	DeviceInfo* d = nullptr;
 	phe_status s = device_info(&d);
 	if (s) return s;
-	*counter = d->counterPool + g_counterNext.fetch_add(1) % kCounterPool;
-	return clear_counter(stream, *counter, early);
+	uint32_t slot = g_counterNext.fetch_add(1) % kCounterPool;
+	uint32_t* c = d->counterPool + slot;
+	*early = !stream_captures(stream);
+	if (*early) {
+		clear_counter_kernel<<<1, 1, 0, stream>>>(c);
+		PHE_CUDA_TRY(cudaGetLastError(), "clear_counter_kernel launch");
+	} else {
+		PHE_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(uint32_t), stream), "cudaMemsetAsync(counter)");
+	}
+	*counter = c;
+	return PHE_OK;
 }
 
 } // namespace phe_gb300

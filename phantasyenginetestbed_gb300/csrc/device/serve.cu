@@ -209,6 +209,7 @@ phe_status launch_wave(phe_server* s, Wave& w, const std::vector<Request*>& item
 	cudaStream_t st = s->waveStream;
 	PHE_CUDA_TRY(cudaMemcpyAsync(w.devItems, w.hostItems, n * sizeof(BatchItemDev), cudaMemcpyHostToDevice, st),
 	             "upload wave table");
+	PHE_CUDA_TRY(cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), st), "clear wave counter");
 	phe_status ps = launch_batch_table(w.devItems, n, base, s->dScenes, w.counter, 128, 0, st, wide);
 	if (ps) return ps;
 	for (uint32_t i = 0; i < n; i++) {
