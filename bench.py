@@ -1003,14 +1003,14 @@ def measure_large(res_side, N, steps, warmup, layout_names=("binary", "wide4", "
                 fn()
             t = _timed(fn, max(3, min(steps, 20)), stream, flush)
             m = statistics.median(t)
-            row[pas] = {"ms": round(m, 3), "Mrays_s": round(N / m / 1e3, 1), "latency_ms": _percentiles(t)}
+            row[pas] = {"ms": round(m, 4), "Mrays_s": round(N / m / 1e3, 1), "latency_ms": _percentiles(t)}
         layouts[name] = row
     scene.set_layout(0)
     torch.cuda.synchronize()
     line = {"workload": "large", "metric": METRIC, "unit": "Mrays/s", "triangles": int(len(s.tri_verts)),
             "bvh_builder": "this project's SBVH builder", "bvh_nodes": int(len(b.nodes)), "bvh_slots": int(len(b.verts)),
             "sbvh_build_s": round(build_s, 1), "scene_bytes": scene.device_bytes(),
-            "primary": {"res": res, "rays": npix, "hits": int(H), "ms": round(t_prim, 3),
+            "primary": {"res": res, "rays": npix, "hits": int(H), "ms": round(t_prim, 4),
                         "Mrays_s": round(npix / t_prim / 1e3, 1)},
             "rays_per_launch": N, "lights": 4, "layouts": layouts,
             "l2": "flushed (512 MiB write) before every timed launch"}
