@@ -55,7 +55,7 @@ __device__ __forceinline__ uint32_t find_item(const BatchItemDev* __restrict__ i
 // status word of the item's scene, which phe_scene_status reads.
 constexpr int kBatchThreadsPerSM = 1280;
 template <int BLOCK, bool WIDE, int SN>
-__global__ void __launch_bounds__(BLOCK, kBatchThreadsPerSM / BLOCK) batch_kernel(BatchTableDev t, uint32_t* __restrict__ counter)
+__global__ void __launch_bounds__(BLOCK, (WIDE ? 128 * kWideMinBlocks : kBatchThreadsPerSM) / BLOCK) batch_kernel(BatchTableDev t, uint32_t* __restrict__ counter)
 {
 	const uint32_t lane = threadIdx.x & 31u;
 	for (;;) {

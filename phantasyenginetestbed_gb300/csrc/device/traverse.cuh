@@ -147,6 +147,7 @@ constexpr int kSmemStack = PHE_SMEM_STACK;
 // Resident blocks of 128 per SM asked for where the 4- and 8-wide traversals are compiled in (72 registers): at 48
 // registers they spill 150 to 440 bytes. 1M diffuse rays on 155K triangles at 7 / 8 / 9 / 10 blocks: 8-wide plain
 // 884 / 934 / 1,004 / 1,025 us, 4-wide 392 / 385 / 374 / 387; an 8-wide 720p frame 893 us at 7, 921 at 8, 972 at 10.
+// 32 batches of up to 256K rays: 4-wide 506 -> 474 us, 8-wide 826 -> 758.
 constexpr int kWideMinBlocks = 7;
 static_assert(kSmemStack >= 0 && kSmemStack <= kStackSize, "shared stack depth");
 extern __shared__ int32_t g_stackSmem[];
