@@ -104,7 +104,8 @@ ChildRef binary_child(const std::vector<float4>& dn, uint32_t node, int c)
 // Moves the tree's upper nodes to the front of the traversal layout `dn`: the kTopNodes with the largest
 // boxes, taken best first from the root (a child never precedes its parent, and the likelier a random
 // ray visits a node, the earlier it comes). A launch of few rays copies them to shared memory. The
-// others keep their order. Child references follow; nothing else depends on a node's index.
+// others keep their order. Child references follow; nothing else depends on a node's index. A node that the
+// root does not reach was not validated and may refer to anything: what is no node's index is left as it is.
 uint32_t move_top_nodes(std::vector<float4>& dn, uint32_t numNodes)
 {
 	auto area = [](const ChildRef& c) {
@@ -139,7 +140,7 @@ uint32_t move_top_nodes(std::vector<float4>& dn, uint32_t numNodes)
 		std::copy_n(&dn[(size_t)order[k] * 4], 4, &out[(size_t)k * 4]);
 		int32_t* iv = reinterpret_cast<int32_t*>(&out[(size_t)k * 4 + 3]);
 		for (int c = 0; c < 2; c++)
-			if (iv[c] >= 0) iv[c] = (int32_t)at[iv[c]];
+			if ((uint32_t)iv[c] < numNodes) iv[c] = (int32_t)at[iv[c]];   // a leaf (~first) is above any index
 	}
 	dn.swap(out);
 	return numTop;

@@ -1,0 +1,102 @@
+"""Host code around the device (scene upload, launch sequences) run without one: the library's own objects
+linked with a CUDA runtime that keeps device memory on the host and records kernels instead of running them
+(tests/cpp/fake_cudart.cpp). Each case runs in a process of its own."""
+import ctypes as C
+import multiprocessing
+import os
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+import phantasyenginetestbed_gb300 as P
+from phantasyenginetestbed_gb300 import build as B
+from phantasyenginetestbed_gb300 import native
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def fake_library(tmp_path_factory):
+    B.build()
+    out = tmp_path_factory.mktemp("fake") / "libphe_fake.so"
+    objects = [str(B.BUILD / f"{s.stem}{s.suffix}.o") for group in B.sources() for s in group]
+    subprocess.run([os.environ.get("CXX", "g++"), "-O1", "-fPIC", "-shared", "-std=c++17", f"-I{B._cuda_include()}",
+                    "-Wl,-Bsymbolic", "-Wl,-z,lazy", "-o", str(out), str(ROOT / "tests/cpp/fake_cudart.cpp"), *objects,
+                    "-lpthread", "-ldl"], check=True)
+    return str(out)
+
+
+def _in_child(case, *args):
+    p = multiprocessing.get_context("spawn").Process(target=case, args=args)
+    p.start()
+    p.join(120)
+    assert p.exitcode == 0, f"exit code {p.exitcode}"
+
+
+def _use(library):
+    """Makes the package of this process use the library with the recording runtime."""
+    lib = C.CDLL(library, mode=os.RTLD_LAZY)
+    for name, (res, args) in native.SIGNATURES.items():
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args
+    lib.fake_allocation.restype = C.c_void_p
+    lib.fake_launch.restype = C.c_char_p
+    native._lib = lib
+    return lib
+
+
+def _allocation(lib, i):
+    size = C.c_size_t()
+    address = lib.fake_allocation(i, C.byref(size))
+    return np.frombuffer(C.string_at(address, size.value), np.uint8)
+
+
+def _upload(lib, nodes, verts):
+    """The bytes of the device nodes and of the rest of the scene's allocation."""
+    scene = P.Scene(nodes, verts)
+    data = _allocation(lib, lib.fake_num_allocations() - 1)
+    scene.close()
+    return data[:64 * len(nodes)], data[(64 * len(nodes) + 255) // 256 * 256:]
+
+
+def _reached(nodes):
+    """The tree that the root of device nodes reaches, depth first, without the numbers of its nodes."""
+    n = nodes.view(np.int32).reshape(-1, 16)
+    out, stack = [], [0]
+    while stack:
+        node = n[stack.pop()].copy()
+        inner = np.nonzero(node[12:14] >= 0)[0] + 12
+        stack += list(node[inner])
+        node[inner] = 0
+        out.append(node)
+    return np.array(out)
+
+
+def _unreached_nodes(library, last):
+    lib = _use(library)
+    b = P.build_sbvh(P.generate_scene(64, 100, False, 7).tri_verts)
+    assert len(b.nodes) > 2048   # some nodes stay behind the ones moved to the front
+    stray = np.zeros(3, P.NODE_DTYPE)
+    stray["iData"] = [[0x10000000, 0x7FFFFFFF, 0, 0], [len(b.nodes) + 2, len(b.nodes) + 3, 0, 0], [-5, 3, 0, 1 << 30]]
+    stray["fData"] = np.nan
+    if last:
+        nodes = np.concatenate([b.nodes, stray])
+    else:   # behind the root: the reached nodes' references move with them
+        nodes = np.concatenate([b.nodes[:1], stray, b.nodes[1:]])
+        reached = np.r_[0, 4:len(nodes)]
+        for c in (0, 1):
+            inner = reached[nodes["iData"][reached, 2 + c] == 0]
+            nodes["iData"][inner, c] += 3
+    want_nodes, want_rest = _upload(lib, b.nodes, b.verts)
+    got_nodes, got_rest = _upload(lib, nodes, b.verts)
+    assert np.array_equal(got_rest, want_rest)
+    assert np.array_equal(_reached(got_nodes), _reached(want_nodes))
+
+
+@pytest.mark.parametrize("last", [True, False])
+def test_upload_ignores_unreached_nodes(fake_library, last):
+    """Nodes that the root does not reach are not validated: whatever they refer to, the upload is that of the tree
+    without them."""
+    _in_child(_unreached_nodes, fake_library, last)
