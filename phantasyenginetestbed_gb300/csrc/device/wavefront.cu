@@ -655,7 +655,7 @@ taa_kernel(uint32_t W, uint32_t H, const float4* __restrict__ cur, const float4*
            float4* __restrict__ outColor, float4* __restrict__ outHist)
 {
 	uint32_t x = blockIdx.x * kTaaBlockX + threadIdx.x;
-	uint32_t y = blockIdx.y * kTaaBlockY + threadIdx.y;
+	uint32_t y = (blockIdx.z * gridDim.y + blockIdx.y) * kTaaBlockY + threadIdx.y;
 	if (x >= W || y >= H) return;
 	size_t p = (size_t)y * W + x;
 	float4 oc, oh;
@@ -838,7 +838,9 @@ extern "C" phe_status phe_taa_resolve(uint32_t resX, uint32_t resY, const float*
 	if (!cur || !hist || !outColor || !outHist) return fail(PHE_ERR_INVALID_ARGUMENT, "phe_taa_resolve: null buffer");
 	if (resX == 0 || resY == 0) return PHE_OK;
 	dim3 block(kTaaBlockX, kTaaBlockY);
-	dim3 grid((resX + kTaaBlockX - 1) / kTaaBlockX, (resY + kTaaBlockY - 1) / kTaaBlockY);
+	// A grid has 65,535 blocks along y, 262,140 rows: a higher image's are split between y and z, up to 524,280 rows.
+	const uint32_t rowBlocks = (resY - 1) / kTaaBlockY + 1, split = rowBlocks > 65535u ? 2u : 1u;
+	dim3 grid((resX - 1) / kTaaBlockX + 1, (rowBlocks - 1) / split + 1, split);
 	// The history and the velocities may be aligned to floats only.
 	const bool vec = !((uintptr_t)hist & 15u) && !((uintptr_t)velocity & 7u) && !((uintptr_t)prevVelocity & 7u);
 	auto kernel = velocity ? (vec ? taa_kernel<true, true> : taa_kernel<false, true>)

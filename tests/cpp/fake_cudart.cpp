@@ -36,7 +36,15 @@ std::map<const void*, std::string>& kernel_names()
 	static std::map<const void*, std::string> names;
 	return names;
 }
-void record(const void* f, dim3 grid, dim3 block, cudaStream_t s, bool early) { g_launches.push_back({kernel_names()[f], grid, block, s, early}); }
+cudaError_t g_lastError = cudaSuccess;
+
+cudaError_t record(const void* f, dim3 grid, dim3 block, cudaStream_t s, bool early)
+{
+	if (!grid.x || !grid.y || !grid.z || grid.x > 0x7FFFFFFFu || grid.y > 65535u || grid.z > 65535u)
+		return g_lastError = cudaErrorInvalidConfiguration;
+	g_launches.push_back({kernel_names()[f], grid, block, s, early});
+	return cudaSuccess;
+}
 
 } // namespace
 
@@ -46,10 +54,11 @@ extern "C" {
 void fake_set_device(int device) { g_device = device; }
 void fake_set_occupancy(int device, int blocks) { g_occupancy[device] = blocks; }
 int fake_num_launches() { return (int)g_launches.size(); }
-const char* fake_launch(int i, uint32_t grid[3], int* early)
+const char* fake_launch(int i, uint32_t grid[3], uint32_t block[3], int* early)
 {
 	const Launch& l = g_launches[i];
 	grid[0] = l.grid.x, grid[1] = l.grid.y, grid[2] = l.grid.z;
+	block[0] = l.block.x, block[1] = l.block.y, block[2] = l.block.z;
 	*early = l.early;
 	return l.kernel.c_str();
 }
@@ -86,8 +95,7 @@ cudaError_t __cudaGetKernel(void** handle, const void* f)
 }
 cudaError_t __cudaLaunchKernel(void* handle, dim3 grid, dim3 block, void**, size_t, cudaStream_t s)
 {
-	record(handle, grid, block, s, false);
-	return cudaSuccess;
+	return record(handle, grid, block, s, false);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**)
 {
@@ -95,8 +103,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 	for (unsigned i = 0; i < c->numAttrs; i++)
 		early = early || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
 		                  c->attrs[i].val.programmaticStreamSerializationAllowed);
-	record(f, c->gridDim, c->blockDim, c->stream, early);
-	return cudaSuccess;
+	return record(f, c->gridDim, c->blockDim, c->stream, early);
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t)
 {
@@ -118,7 +125,12 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int)
 	return cudaSuccess;
 }
 const char* cudaGetErrorString(cudaError_t) { return "error"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+	const cudaError_t e = g_lastError;
+	g_lastError = cudaSuccess;
+	return e;
+}
 cudaError_t cudaMalloc(void** p, size_t n)
 {
 	const size_t size = (n + 255) & ~size_t(255);

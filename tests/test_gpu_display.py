@@ -89,3 +89,21 @@ def test_taa_without_velocities(res, shift):
         want_c, want_h = O.taa(cur, hist, rough, zero, zero if prev is None else prev)
         assert np.array_equal(from_device(oc, np.float32).reshape(H, W, 4), want_c)
         assert np.array_equal(from_device(oh, np.float32).reshape(H, W, 4), want_h)
+
+
+@pytest.mark.parametrize("moving", [False, True])
+@pytest.mark.parametrize("rows", [262140, 262141, 262149, 524280])   # the last of one block per grid row, then two
+def test_taa_of_high_images(rows, moving):
+    import torch
+    W = 2
+    rng = np.random.default_rng(rows)
+    cur, hist = (rng.uniform(0, 2, (rows, W, 4)).astype(np.float32) for _ in range(2))
+    vel = (rng.normal(size=(rows, W, 2)) * 1e-5).astype(np.float32) if moving else None
+    rough = rng.uniform(0, 1, (rows, W)).astype(np.float32)
+    oc, oh = (device_empty(W * rows, np.dtype((np.float32, 4))) for _ in range(2))
+    taa_resolve((W, rows), to_device(cur), to_device(hist), oc, oh, to_device(vel) if moving else None, None, to_device(rough))
+    torch.cuda.synchronize()
+    want_c, want_h = O.taa(cur, hist, rough, np.zeros((rows, W, 2), np.float32) if vel is None else vel,
+                           np.zeros((rows, W, 2), np.float32))
+    assert np.array_equal(from_device(oc, np.float32).reshape(rows, W, 4), want_c)
+    assert np.array_equal(from_device(oh, np.float32).reshape(rows, W, 4), want_h)

@@ -53,6 +53,16 @@ def _allocation(lib, i):
     return np.frombuffer(C.string_at(address, size.value), np.uint8)
 
 
+def _launches(lib):
+    """Every launch so far: kernel, grid, block, whether it may start early."""
+    out = []
+    for i in range(lib.fake_num_launches()):
+        grid, block, early = (C.c_uint32 * 3)(), (C.c_uint32 * 3)(), C.c_int()
+        name = lib.fake_launch(i, grid, block, C.byref(early)).decode()
+        out.append((name, tuple(grid), tuple(block), bool(early.value)))
+    return out
+
+
 def _upload(lib, nodes, verts):
     """The bytes of the device nodes and of the rest of the scene's allocation."""
     scene = P.Scene(nodes, verts)
@@ -100,3 +110,19 @@ def test_upload_ignores_unreached_nodes(fake_library, last):
     """Nodes that the root does not reach are not validated: whatever they refer to, the upload is that of the tree
     without them."""
     _in_child(_unreached_nodes, fake_library, last)
+
+
+def _taa_heights(library):
+    lib = _use(library)
+    buf = C.c_void_p(1 << 20)
+    for h in (1, 4, 5, 262140, 262141, 262149, 524279, 524280):
+        assert lib.phe_taa_resolve(40, h, buf, buf, None, None, None, buf, buf, None) == native.PHE_OK, h
+        name, grid, block, _ = _launches(lib)[-1]
+        assert "taa_kernel" in name and grid[0] * block[0] >= 40 and grid[1] * grid[2] * block[1] >= h
+    n = lib.fake_num_launches()
+    assert lib.phe_taa_resolve(40, 524281, buf, buf, None, None, None, buf, buf, None) == native.PHE_ERR_CUDA
+    assert lib.fake_num_launches() == n
+
+
+def test_taa_takes_images_up_to_524280_rows(fake_library):
+    _in_child(_taa_heights, fake_library)
