@@ -78,6 +78,7 @@ constexpr int32_t kSentinel = 0x7FFFFFFF;
 constexpr uint32_t kErrStackOverflow = 1u;
 constexpr uint32_t kErrBadIndex = 2u;   // checked build: a node or slot index outside its array
 constexpr uint32_t kErrTopCopy = 4u;    // a block's copy of the upper nodes did not arrive in time (it read global memory)
+constexpr uint32_t kErrCopyPending = 8u;   // and had not when the block ended: it may have written another block's shared memory
 
 // The checked build (-DPHE_DEVICE_CHECKS=1, libphe_gb300_checked.so) tests every node and slot index a
 // traversal is about to read against the array sizes; an index outside sets kErrBadIndex and ends that

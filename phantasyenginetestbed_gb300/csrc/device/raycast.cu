@@ -12,6 +12,7 @@
 #include <atomic>
 
 #include "runtime.cuh"
+#include "small_cast.cuh"
 #include "traverse.cuh"
 
 namespace phe_gb300 {
@@ -71,67 +72,6 @@ __global__ void __launch_bounds__(kPersistentBlock, cast_min_blocks(WIDE)) close
 		}
 		__syncwarp();
 		base = next_rays(counter);
-	}
-}
-
-// Launches of few rays (small_cast below): every chunk of rays has a warp from the start, so there is no
-// work counter to clear, and one block an SM spreads the warps over the chip.
-//
-// Such a launch lasts as long as its slowest warp, whose loads no other warp hides: the tree's upper
-// nodes (numTop of them, at most 128 KB) come to shared memory in bulk copies while the rays load, a
-// leaf's triangles are loaded three at a time, and registers are plentiful. 4,096 rays on 10K
-// triangles: closest hit 58 -> 52 us; any hit 51.5 -> 34 us, with 4 rays a warp (below).
-constexpr int kSmallMaxWarps = 16;
-constexpr int kSmallLeaf = 3;
-constexpr int kCopyWaits = 1 << 20;   // bound of the wait for the copy (each try waits some time itself)
-
-__device__ __forceinline__ bool wait_copy(uint32_t barrier)
-{
-	uint32_t done = 0;
-	for (int k = 0; k < kCopyWaits && !done; k++)
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-		             : "=r"(done) : "r"(barrier) : "memory");
-	return done != 0;
-}
-
-template <bool ANY>
-__global__ void __launch_bounds__(32 * kSmallMaxWarps, 1)
-small_cast_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays, void* __restrict__ out, const uint32_t* __restrict__ scatter,
-                  uint32_t n, uint32_t numTop, uint32_t raysPerWarp, uint32_t* __restrict__ status)
-{
-	extern __shared__ ulonglong2 topNodes[];
-	__shared__ alignas(8) unsigned long long barrierWord;
-	const uint32_t barrier = (uint32_t)__cvta_generic_to_shared(&barrierWord);
-	if (threadIdx.x == 0) {
-		const uint32_t bytes = numTop * 64u, dst = (uint32_t)__cvta_generic_to_shared(topNodes);
-		asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(barrier));
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-		asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(barrier), "r"(bytes) : "memory");
-		for (uint32_t at = 0; at < bytes; at += 16384u)
-			asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + at),
-			             "l"((const char*)s.nodes + at), "r"(min(16384u, bytes - at)), "r"(barrier)
-			             : "memory");
-	}
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t i = (blockIdx.x + gridDim.x * (threadIdx.x >> 5)) * raysPerWarp + lane;
-	const bool active = lane < raysPerWarp && i < n;
-	RayState r;
-	if (active) r = load_ray(rays, i);
-	__syncthreads();   // the barrier is initialised
-	const bool copied = wait_copy(barrier);
-	if (active) {
-		HitRecord h = empty_hit(r);
-		const TraversalBounds bd{s.numNodes, s.numSlots};
-		const TopNodes nodes{s.nodes, topNodes, copied ? numTop : 0u};
-		const uint32_t err = fast_ray(r, s.dirLimit) ? traverse<true, ANY, 0, kSmallLeaf>(nodes, s.tris, bd, r, h)
-		                                             : traverse<false, ANY, 0, kSmallLeaf>(nodes, s.tris, bd, r, h);
-		if (err) atomicOr(status, err);
-		if (ANY) ((uint8_t*)out)[scatter ? __ldg(scatter + i) : i] = h.slot == ~0u ? 1 : 0;
-		else store_hit((phe_ray_hit*)out, i, r, h);
-	}
-	if (!copied) {   // the copy still writes this block's shared memory
-		if (threadIdx.x == 0) atomicOr(status, kErrTopCopy);
-		wait_copy(barrier);
 	}
 }
 
@@ -218,7 +158,8 @@ static phe_status small_cast(const phe_scene* scene, const phe_ray_in* rays, voi
 		             "small_cast_kernel shared memory");
 		sized.fetch_or(uint64_t(1) << d->device, std::memory_order_relaxed);
 	}
-	kernel<<<grid, 32 * perBlock, smem, stream>>>(scene->dev, rays, out, scatter, n, scene->dev.numTop, perWarp, scene->status);
+	kernel<<<grid, 32 * perBlock, smem, stream>>>(scene->dev, rays, out, scatter, n, scene->dev.numTop, perWarp, kCopyWaits,
+	                                           scene->status);
 	PHE_CUDA_TRY(cudaGetLastError(), "small_cast_kernel launch");
 	*done = true;
 	return PHE_OK;
