@@ -88,18 +88,19 @@ __global__ void __launch_bounds__(BLOCK, (WIDE ? 128 * kWideMinBlocks : kBatchTh
 // `wide` selects the instantiation with the 4-wide traversal (for scene tables holding 4-wide scenes),
 // `stackShared` (0 or kBatchStackShared) the one keeping that many stack entries in shared memory.
 template <int BLOCK>
-static phe_status launch_batch_kernel(const BatchTableDev& t, bool wide, int stackShared, int blocksPerSM, int numSMs,
+static phe_status launch_batch_kernel(const BatchTableDev& t, bool wide, int stackShared, int blocksPerSM, const DeviceInfo& d,
                                       uint32_t* counter, cudaStream_t stream, int* occupancyOut)
 {
 	const bool sh = stackShared > 0;
 	auto kernel = wide ? (sh ? batch_kernel<BLOCK, true, kBatchStackShared> : batch_kernel<BLOCK, true, 0>)
 	                   : (sh ? batch_kernel<BLOCK, false, kBatchStackShared> : batch_kernel<BLOCK, false, 0>);
 	const size_t smem = stack_smem_bytes(BLOCK, sh ? kBatchStackShared : 0);
-	static std::atomic<int> occupancy[2][2] = {};   // [wide][sh]; filled on first use (threads that race store the same value)
-	int maxB = occupancy[wide][sh].load(std::memory_order_relaxed);
+	static std::atomic<int> occupancy[kMaxDevices][2][2] = {};   // [device][wide][sh]; filled on first use (threads that race store the same value)
+	std::atomic<int>& known = occupancy[d.device][wide][sh];
+	int maxB = known.load(std::memory_order_relaxed);
 	if (maxB == 0) {
 		PHE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxB, kernel, BLOCK, smem), "occupancy");
-		occupancy[wide][sh].store(maxB, std::memory_order_relaxed);
+		known.store(maxB, std::memory_order_relaxed);
 	}
 	if (occupancyOut) {
 		*occupancyOut = maxB;
@@ -107,7 +108,7 @@ static phe_status launch_batch_kernel(const BatchTableDev& t, bool wide, int sta
 	}
 	int b = blocksPerSM > 0 ? std::min(blocksPerSM, maxB) : maxB;
 	if (b < 1) b = 1;
-	uint32_t grid = (uint32_t)(b * numSMs);
+	uint32_t grid = (uint32_t)(b * d.numSMs);
 	uint32_t need = (t.totalPadded + BLOCK - 1) / BLOCK;
 	if (grid > need) grid = need > 0 ? need : 1;
 	kernel<<<grid, BLOCK, smem, stream>>>(t, counter);
@@ -157,9 +158,9 @@ phe_status launch_batch_table(const BatchItemDev* items, uint32_t numItems, uint
 	if (totalPadded == 0) return PHE_OK;
 	BatchTableDev t{items, scenes, numItems, totalPadded, nullptr};
 	switch (blockSize) {
-	case 64: return launch_batch_kernel<64>(t, wide, 0, blocksPerSM, d->numSMs, counter, stream, nullptr);
-	case 256: return launch_batch_kernel<256>(t, wide, 0, blocksPerSM, d->numSMs, counter, stream, nullptr);
-	default: return launch_batch_kernel<128>(t, wide, 0, blocksPerSM, d->numSMs, counter, stream, nullptr);
+	case 64: return launch_batch_kernel<64>(t, wide, 0, blocksPerSM, *d, counter, stream, nullptr);
+	case 256: return launch_batch_kernel<256>(t, wide, 0, blocksPerSM, *d, counter, stream, nullptr);
+	default: return launch_batch_kernel<128>(t, wide, 0, blocksPerSM, *d, counter, stream, nullptr);
 	}
 }
 
@@ -405,9 +406,9 @@ static phe_status batch_enqueue(phe_batch* b, cudaStream_t stream)
 	const bool wide = b->params.layout == PHE_LAYOUT_WIDE4 || b->params.layout == PHE_LAYOUT_WIDE8;
 	const int sh = b->params.stackShared;
 	switch (b->params.blockSize) {
-	case 64: return launch_batch_kernel<64>(t, wide, sh, b->params.blocksPerSM, d->numSMs, b->dCounter, stream, nullptr);
-	case 256: return launch_batch_kernel<256>(t, wide, sh, b->params.blocksPerSM, d->numSMs, b->dCounter, stream, nullptr);
-	case 128: return launch_batch_kernel<128>(t, wide, sh, b->params.blocksPerSM, d->numSMs, b->dCounter, stream, nullptr);
+	case 64: return launch_batch_kernel<64>(t, wide, sh, b->params.blocksPerSM, *d, b->dCounter, stream, nullptr);
+	case 256: return launch_batch_kernel<256>(t, wide, sh, b->params.blocksPerSM, *d, b->dCounter, stream, nullptr);
+	case 128: return launch_batch_kernel<128>(t, wide, sh, b->params.blocksPerSM, *d, b->dCounter, stream, nullptr);
 	default: return fail(PHE_ERR_INVALID_ARGUMENT, "batch block size must be 64, 128 or 256");
 	}
 }
@@ -427,13 +428,15 @@ extern "C" phe_status phe_batch_launch(phe_batch* b, void* stream)
 	if (!b->graph) {
 		// Resolve occupancy outside capture.
 		int occ = 0;
+		DeviceInfo* d = nullptr;
+		if (phe_status st = device_info(&d)) return st;
 		BatchTableDev t{};
 		const bool wide = b->params.layout == PHE_LAYOUT_WIDE4 || b->params.layout == PHE_LAYOUT_WIDE8;
 		const int sh = b->params.stackShared;
 		switch (b->params.blockSize) {
-		case 64: launch_batch_kernel<64>(t, wide, sh, 0, 1, nullptr, nullptr, &occ); break;
-		case 256: launch_batch_kernel<256>(t, wide, sh, 0, 1, nullptr, nullptr, &occ); break;
-		default: launch_batch_kernel<128>(t, wide, sh, 0, 1, nullptr, nullptr, &occ); break;
+		case 64: launch_batch_kernel<64>(t, wide, sh, 0, *d, nullptr, nullptr, &occ); break;
+		case 256: launch_batch_kernel<256>(t, wide, sh, 0, *d, nullptr, nullptr, &occ); break;
+		default: launch_batch_kernel<128>(t, wide, sh, 0, *d, nullptr, nullptr, &occ); break;
 		}
 		cudaStream_t cap = nullptr;
 		PHE_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "create capture stream");
@@ -526,9 +529,9 @@ extern "C" phe_status phe_batch_autotune(phe_batch* b, int repeats, void* stream
 	for (int bs : blocks) {
 		int occ = 0;
 		BatchTableDev t{};
-		if (bs == 64) launch_batch_kernel<64>(t, false, 0, 0, 1, nullptr, nullptr, &occ);
-		else if (bs == 128) launch_batch_kernel<128>(t, false, 0, 0, 1, nullptr, nullptr, &occ);
-		else launch_batch_kernel<256>(t, false, 0, 0, 1, nullptr, nullptr, &occ);
+		if (bs == 64) launch_batch_kernel<64>(t, false, 0, 0, *d, nullptr, nullptr, &occ);
+		else if (bs == 128) launch_batch_kernel<128>(t, false, 0, 0, *d, nullptr, nullptr, &occ);
+		else launch_batch_kernel<256>(t, false, 0, 0, *d, nullptr, nullptr, &occ);
 		for (int ord : orders)
 			for (int q : occFrac)
 				for (int lay : layouts)

@@ -33,6 +33,7 @@ struct DeviceInfo {
 	uint32_t* counterPool = nullptr; // kCounterPool words
 };
 
+constexpr int kMaxDevices = 64;   // device ordinals that the library takes
 constexpr uint32_t kCounterPool = 4096;
 // Largest ray count of one persistent launch. Every resident warp fetches 32 rays past the end before
 // it stops, so the 32-bit work counter needs headroom above the count (2^26 covers 2M resident warps).

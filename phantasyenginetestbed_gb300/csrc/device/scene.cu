@@ -18,7 +18,7 @@
 namespace phe_gb300 {
 
 static std::mutex g_devMutex;
-static DeviceInfo g_devices[64];
+static DeviceInfo g_devices[kMaxDevices];
 static std::atomic<uint32_t> g_counterNext{0};
 
 phe_status device_info(DeviceInfo** out)
@@ -26,7 +26,7 @@ phe_status device_info(DeviceInfo** out)
 	int dev = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess) return fail(PHE_ERR_NO_DEVICE, "no CUDA device: %s", cudaGetErrorString(e));
-	if (dev < 0 || dev >= 64) return fail(PHE_ERR_NO_DEVICE, "device ordinal %d out of range", dev);
+	if (dev < 0 || dev >= kMaxDevices) return fail(PHE_ERR_NO_DEVICE, "device ordinal %d out of range", dev);
 	std::lock_guard<std::mutex> lock(g_devMutex);
 	DeviceInfo& d = g_devices[dev];
 	if (d.device < 0) {

@@ -126,3 +126,23 @@ def _taa_heights(library):
 
 def test_taa_takes_images_up_to_524280_rows(fake_library):
     _in_child(_taa_heights, fake_library)
+
+
+def _batch_grids(library, graph):
+    from phantasyenginetestbed_gb300.batch import Batch
+    lib = _use(library)
+    b = P.build_sbvh(P.generate_scene(8, 2, False, 7).tri_verts)
+    for device, blocks in ((0, 3), (1, 5), (0, 3)):
+        lib.fake_set_device(device)
+        lib.fake_set_occupancy(device, blocks)
+        scene = P.Scene(b.nodes, b.verts)
+        batch = Batch([scene], [(0, 0, 1 << 20, 1 << 20, 2 << 20), (0, 1, 1 << 20, 3 << 20, 4 << 20)], use_graph=graph)
+        batch.launch()
+        name, grid, block, _ = _launches(lib)[-1]
+        assert "batch_kernel" in name and grid == (152 * blocks, 1, 1) and block[0] == 128, (name, grid)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_batch_grid_follows_the_device(fake_library, graph):
+    """The resident blocks that size a batch's grid are those of the device it is launched on."""
+    _in_child(_batch_grids, fake_library, graph)
