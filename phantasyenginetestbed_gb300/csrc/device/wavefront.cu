@@ -734,10 +734,11 @@ phe_status launch_frame(const phe_scene* scene, const FrameParamsDev* dParams, c
 	DeviceInfo* dinfo = nullptr;
 	if ((st = device_info(&dinfo))) return st;
 	int binGrid = dinfo->numSMs * 4;
-	// A stage is queued to start while the one before it ends (launch_early), unless an event is recorded between the
-	// two or the frame goes into a graph, whose own edges measured the same: a 256x256 frame on 10K triangles 129 ->
-	// 121 us, two 256x144 frames in flight 98 -> 94.5 us each on 155K, 0.5-1% at 1080p.
-	const bool early = !ev && !stream_captures(stream);
+	// A stage is queued to start while the one before it ends (launch_early), unless events come between the two (timed
+	// frames, the fork and join of the beside schedule) or the frame goes into a graph, whose own edges measured the
+	// same: a 256x256 frame on 10K triangles 129 -> 121 us, two 256x144 frames in flight 98 -> 94.5 us each on 155K,
+	// 0.5-1% at 1080p.
+	const bool early = !ev && !beside && !stream_captures(stream);
 	if (parts & kFrameTraversal) {
 		mark();
 		if (fused) {

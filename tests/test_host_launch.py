@@ -146,3 +146,32 @@ def _batch_grids(library, graph):
 def test_batch_grid_follows_the_device(fake_library, graph):
     """The resident blocks that size a batch's grid are those of the device it is launched on."""
     _in_child(_batch_grids, fake_library, graph)
+
+
+def _frame_launches(library, schedule, timed, want):
+    from phantasyenginetestbed_gb300 import renderer as R
+    lib = _use(library)
+    s = P.generate_scene(8, 2, False, 7)
+    b = P.build_sbvh(s.tri_verts)
+    r = R.CudaTracerRenderer()
+    r.setStaticScene(P.Scene.from_bvh(b, s))
+    r.setTargetResolution((64, 64))
+    r.set_shadow_schedule(schedule)
+    r.set_kernel_timing(timed)
+    r.updateCamera((0.5, -0.3, 0.6), (0.0, 0.8, -0.6), (0.0, 0.6, 0.8), 60.0)
+    n = lib.fake_num_launches()
+    r.render(R.make_lights(np.array([[0.1, 0.1, 0.5]], np.float32), range_=100.0))
+    got = [(k, early) for name, _, _, early in _launches(lib)[n:]
+           for k in ("primary", "any_queue", "bounce", "resolve_taa") if k + "_kernel" in name]
+    assert got == want, got
+
+
+@pytest.mark.parametrize("schedule,timed,want", [
+    (2, False, [("primary", False), ("bounce", True), ("any_queue", True), ("resolve_taa", True)]),
+    (2, True, [("primary", False), ("bounce", False), ("any_queue", False), ("resolve_taa", False)]),
+    (0, False, [("primary", False), ("any_queue", False), ("bounce", True), ("any_queue", False), ("resolve_taa", True)]),
+    (1, False, [("primary", False), ("any_queue", False), ("bounce", False), ("any_queue", False), ("resolve_taa", False)])])
+def test_stages_start_early_only_behind_a_kernel(fake_library, schedule, timed, want):
+    """A frame stage is launched early only where the kernel before it is the stream's last work: not behind the events
+    of a timed frame, nor behind the fork and the join of the beside schedule (1)."""
+    _in_child(_frame_launches, fake_library, schedule, timed, want)
