@@ -14,7 +14,7 @@ __device__ __forceinline__ float glsl_mix(float a, float b, float t)
 }
 
 // One axis of GL_LINEAR with clamp to edge: the two texels around pixel-space position p (texel centres at
-// integer + 0.5) of n, and the weight of the second.
+// integer + 0.5) of n (1 to 2^32 - 1), and the weight of the second.
 struct LinearAxis {
 	uint32_t i0, i1;
 	float a;
@@ -22,11 +22,11 @@ struct LinearAxis {
 __device__ __forceinline__ LinearAxis linear_axis(float p, uint32_t n)
 {
 	const float f = __fsub_rn(p, 0.5f), f0 = floorf(f);
-	const int i = (int)f0, m = (int)n - 1;   // images are at most 65536 texels wide and high
+	const uint32_t m = n - 1;
 	LinearAxis r;
 	r.a = __fsub_rn(f, f0);
-	r.i0 = (uint32_t)min(max(i, 0), m);
-	r.i1 = (uint32_t)min(max(i == 0x7FFFFFFF ? i : i + 1, 0), m);
+	r.i0 = min(__float2uint_rz(f0), m);   // the conversion saturates: 0 below the first texel
+	r.i1 = min(r.i0 + (f0 >= 0.0f ? 1u : 0u), m);
 	return r;
 }
 

@@ -23,6 +23,14 @@ def test_filmic_curve_is_the_divided_one(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_linear_axis_of_any_size(tmp_path):
+    out = tmp_path / "sampling_test"
+    subprocess.run([B._nvcc(), *B.ARCH, "-std=c++17", "-fmad=false", f"-I{ROOT / 'include'}", f"-I{B.CSRC / 'device'}",
+                    str(ROOT / "tests/cpp/sampling_test.cu"), "-o", str(out)], check=True)
+    r = subprocess.run([str(out)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def _floats(a, shift):
     """`a` on the device, `shift` floats past an aligned address."""
     import torch
