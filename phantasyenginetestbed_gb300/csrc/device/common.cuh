@@ -63,7 +63,7 @@ struct DeviceScene {
 };
 static_assert(sizeof(DeviceScene) == 128, "DeviceScene is 128 bytes");
 
-// Nodes that move_top_nodes (scene.cu) puts first.
+// Nodes that place_nodes (scene.cu) puts first.
 constexpr uint32_t kTopNodes = 2048;
 constexpr int32_t kEmptyChild = 0x7FFFFFFE;
 

@@ -101,62 +101,42 @@ ChildRef binary_child(const std::vector<float4>& dn, uint32_t node, int c)
 	return r;
 }
 
-// Moves the tree's upper nodes to the front of the traversal layout `dn`: the kTopNodes with the largest
+// Where each node goes in the traversal layout: the tree's upper nodes first, the kTopNodes with the largest
 // boxes, taken best first from the root (a child never precedes its parent, and the likelier a random
 // ray visits a node, the earlier it comes). A launch of few rays copies them to shared memory. The
-// others keep their order. Child references follow; nothing else depends on a node's index. A node that the
-// root does not reach was not validated and may refer to anything: what is no node's index is left as it is.
-uint32_t move_top_nodes(std::vector<float4>& dn, uint32_t numNodes)
+// others keep their order; nothing depends on a node's index. Returns the number of upper nodes.
+uint32_t place_nodes(const std::vector<phe_bvh_node>& nodes, std::vector<uint32_t>& at)
 {
-	auto area = [](const ChildRef& c) {
-		const float x = c.box[3] - c.box[0], y = c.box[4] - c.box[1], z = c.box[5] - c.box[2];
-		return x * y + y * z + z * x;
-	};
-	std::vector<uint32_t> order;
-	std::vector<uint8_t> moved(numNodes, 0);
-	order.reserve(numNodes);
+	constexpr uint32_t kOther = 0xFFFFFFFFu;
+	at.assign(nodes.size(), kOther);
 	std::priority_queue<std::pair<float, uint32_t>> open;
 	open.push({std::numeric_limits<float>::infinity(), 0u});
-	while (!open.empty() && order.size() < kTopNodes) {
-		const uint32_t n = open.top().second;
+	uint32_t numTop = 0;
+	while (!open.empty() && numTop < kTopNodes) {
+		const phe_bvh_node& n = nodes[open.top().second];
+		at[open.top().second] = numTop++;
 		open.pop();
-		moved[n] = 1;
-		order.push_back(n);
 		for (int c = 0; c < 2; c++) {
-			const ChildRef ch = binary_child(dn, n, c);
-			if (ch.ref >= 0) {
-				const float a = area(ch);
-				open.push({std::isnan(a) ? 0.0f : a, (uint32_t)ch.ref});
-			}
+			if (n.iData[2 + c] > 0) continue;
+			const float* b = n.fData + 6 * c;   // lo.xyz, hi.xyz
+			const float x = b[3] - b[0], y = b[4] - b[1], z = b[5] - b[2], area = x * y + y * z + z * x;
+			open.push({std::isnan(area) ? 0.0f : area, (uint32_t)n.iData[c]});
 		}
 	}
-	const uint32_t numTop = (uint32_t)order.size();
-	for (uint32_t n = 0; n < numNodes; n++)
-		if (!moved[n]) order.push_back(n);
-	std::vector<uint32_t> at(numNodes);
-	for (uint32_t k = 0; k < numNodes; k++) at[order[k]] = k;
-	std::vector<float4> out(dn.size());
-	for (uint32_t k = 0; k < numNodes; k++) {
-		std::copy_n(&dn[(size_t)order[k] * 4], 4, &out[(size_t)k * 4]);
-		int32_t* iv = reinterpret_cast<int32_t*>(&out[(size_t)k * 4 + 3]);
-		for (int c = 0; c < 2; c++)
-			if ((uint32_t)iv[c] < numNodes) iv[c] = (int32_t)at[iv[c]];   // a leaf (~first) is above any index
-	}
-	dn.swap(out);
+	uint32_t next = numTop;
+	for (uint32_t& k : at)
+		if (k == kOther) k = next++;
 	return numTop;
 }
 
 // Largest ray-direction component D for which |det| = |e1 . (d x e2)| <= 6 D E^2 stays below 2^126 (E: the
-// largest edge component of the slots `dt`), with a factor of four to spare for rounding; -1 (no
+// largest edge component, as the bits of its magnitude), with a factor of four to spare for rounding; -1 (no
 // direction) when an edge is not finite.
-float direction_limit(const std::vector<float4>& dt)
+float direction_limit(uint32_t largestEdgeBits)
 {
-	float e = 0.0f;
-	for (size_t i = 0; i < dt.size(); i += 3)
-		for (float x : {dt[i + 1].x, dt[i + 1].y, dt[i + 1].z, dt[i + 1].w, dt[i + 2].x, dt[i + 2].y}) {
-			if (!std::isfinite(x)) return -1.0f;
-			e = std::max(e, std::fabs(x));
-		}
+	float e;
+	std::memcpy(&e, &largestEdgeBits, sizeof(e));
+	if (!std::isfinite(e)) return -1.0f;
 	const double limit = 0x1p124 / (6.0 * (double)e * (double)e);
 	return (float)std::min(limit, (double)3.402823466e+38f);
 }
@@ -368,9 +348,11 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	std::vector<float4> dn((size_t)numNodes * 4);
 	std::vector<float4> dt(((size_t)numSlots + kTriPadding) * 3);
 	std::vector<uint8_t> used(numSlots, 0);
+	std::vector<uint32_t> at;
+	const uint32_t numTop = place_nodes(hn, at);
 	for (uint32_t i = 0; i < numNodes; i++) {
 		const phe_bvh_node& n = hn[i];
-		float4* o = &dn[(size_t)i * 4];
+		float4* o = &dn[(size_t)at[i] * 4];
 		const float *b0 = n.fData, *b1 = n.fData + 6;   // lo.xyz, hi.xyz of each child
 		o[0] = make_float4(b0[0], b0[1], b0[3], b0[4]);
 		o[1] = make_float4(b1[0], b1[1], b1[3], b1[4]);
@@ -383,13 +365,15 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 				int32_t first = raw < 0 ? ~raw : raw;
 				idx[c] = ~first;
 			} else {
-				idx[c] = raw;
+				// A node that the root does not reach was not validated and may refer to anything.
+				idx[c] = (uint32_t)raw < numNodes ? (int32_t)at[raw] : raw;
 				cnt[c] = 0;
 			}
 		}
 		int4 iv = make_int4(idx[0], idx[1], cnt[0], cnt[1]);
 		std::memcpy(&o[3], &iv, sizeof(iv));
 	}
+	uint32_t largestEdge = 0;   // of the edges' components, the bits of the magnitude (NaN above infinity above the rest)
 	for (uint32_t i = 0; i < numSlots; i++) {
 		const phe_triangle_vertices& t = hv[i];
 		float e1x = t.v1[0] - t.v0[0], e1y = t.v1[1] - t.v0[1], e1z = t.v1[2] - t.v0[2];
@@ -398,6 +382,9 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 		o[0] = make_float4(t.v0[0], t.v0[1], t.v0[2], 0.0f);
 		o[1] = make_float4(e2x, e1x, e2y, e1y);
 		o[2] = make_float4(e2z, e1z, 0.0f, 0.0f);
+		uint32_t edges[6];
+		std::memcpy(edges, &o[1], sizeof(edges));
+		for (uint32_t x : edges) largestEdge = std::max(largestEdge, x & 0x7FFFFFFFu);
 	}
 	// End markers from the leaf ranges of the reachable tree (phe_bvh_validate checked the ranges).
 	{
@@ -434,7 +421,6 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 		w8.leaves.clear();
 	}
 
-	const uint32_t numTop = move_top_nodes(dn, numNodes);
 	size_t nodeBytes = align256(dn.size() * sizeof(float4));
 	size_t node4Bytes = align256(dn4.size() * sizeof(float4));
 	size_t node8Bytes = align256(w8.nodes.size() * sizeof(uint32_t));
@@ -495,7 +481,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	sc->maxDepth8 = w8.depth;
 	sc->dev.numNodes8 = sc->numNodes8;
 	sc->dev.numLeaves8 = sc->numLeaves8;
-	sc->dev.dirLimit = direction_limit(dt);
+	sc->dev.dirLimit = direction_limit(largestEdge);
 	sc->dev.numTop = numTop;
 	sc->dev.numNodes4 = (uint32_t)(dn4.size() / 8);
 	sc->maxDepth4 = depth4;
