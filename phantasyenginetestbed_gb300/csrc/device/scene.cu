@@ -8,8 +8,11 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <queue>
+#include <utility>
 #include <vector>
 
 #include "../host/wide8.hpp"
@@ -84,6 +87,12 @@ static_assert(sizeof(phe_ray_hit) == 16, "RayHit is 16 bytes");
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 namespace {
+
+struct DeviceAllocation {   // freed unless released
+	char* p;
+	~DeviceAllocation() { if (p) cudaFree(p); }
+	char* release() { return std::exchange(p, nullptr); }
+};
 
 struct ChildRef {
 	float box[6];   // lo.xyz, hi.xyz
@@ -297,9 +306,9 @@ phe_status upload_shading(phe_scene* sc, const phe_material* mats, uint32_t numM
 
 } // namespace
 
-extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNodes, const phe_triangle_vertices* verts,
-                                       const phe_triangle_data* datas, uint32_t numSlots, const phe_material* materials,
-                                       uint32_t numMaterials, int where, phe_scene** out)
+static phe_status create_scene(const phe_bvh_node* nodes, uint32_t numNodes, const phe_triangle_vertices* verts,
+                               const phe_triangle_data* datas, uint32_t numSlots, const phe_material* materials,
+                               uint32_t numMaterials, int where, phe_scene** out)
 {
 	if (!out) return fail(PHE_ERR_INVALID_ARGUMENT, "phe_scene_create: out is null");
 	NvtxRange range("phe_scene_create");
@@ -319,14 +328,10 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	std::vector<phe_triangle_vertices> hv;
 	std::vector<phe_triangle_data> hd;
 	std::vector<phe_material> hm;
-	try {
-		hn.resize(numNodes);
-		hv.resize(numSlots);
-		if (datas) hd.resize(numSlots);
-		if (materials && numMaterials) hm.resize(numMaterials);
-	} catch (const std::bad_alloc&) {
-		return fail(PHE_ERR_OUT_OF_MEMORY, "phe_scene_create: host staging allocation failed");
-	}
+	hn.resize(numNodes);
+	hv.resize(numSlots);
+	if (datas) hd.resize(numSlots);
+	if (materials && numMaterials) hm.resize(numMaterials);
 	cudaMemcpyKind kind = where == PHE_PTR_HOST ? cudaMemcpyHostToHost : cudaMemcpyDeviceToHost;
 	PHE_CUDA_TRY(cudaMemcpy(hn.data(), nodes, sizeof(phe_bvh_node) * (size_t)numNodes, kind), "copy nodes");
 	PHE_CUDA_TRY(cudaMemcpy(hv.data(), verts, sizeof(phe_triangle_vertices) * (size_t)numSlots, kind), "copy verts");
@@ -432,7 +437,7 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	char* base = nullptr;
 	cudaError_t e = cudaMalloc(&base, total);
 	if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(scene)");
-	auto cleanup = [&](phe_status st) { cudaFree(base); return st; };
+	DeviceAllocation allocation{base};
 	char* p = base;
 	float4* dNodes = (float4*)p; p += nodeBytes;
 	float4* dNodes4 = dn4.empty() ? nullptr : (float4*)p; p += node4Bytes;
@@ -442,21 +447,21 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	phe_triangle_data* dDatas = hd.empty() ? nullptr : (phe_triangle_data*)p; p += dataBytes;
 	uint32_t* dStatus = (uint32_t*)p;
 	if ((e = cudaMemcpy(dNodes, dn.data(), dn.size() * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload nodes"));
+		return cuda_fail(e, "upload nodes");
 	if (dNodes4 && (e = cudaMemcpy(dNodes4, dn4.data(), dn4.size() * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload 4-wide nodes"));
+		return cuda_fail(e, "upload 4-wide nodes");
 	if (dNodes8 && (e = cudaMemcpy(dNodes8, w8.nodes.data(), w8.nodes.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload 8-wide nodes"));
+		return cuda_fail(e, "upload 8-wide nodes");
 	if (dLeaves8 && (e = cudaMemcpy(dLeaves8, w8.leaves.data(), w8.leaves.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload 8-wide leaf records"));
+		return cuda_fail(e, "upload 8-wide leaf records");
 	if ((e = cudaMemcpy(dTris, dt.data(), dt.size() * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload triangles"));
+		return cuda_fail(e, "upload triangles");
 	if (dDatas && (e = cudaMemcpy(dDatas, hd.data(), hd.size() * sizeof(phe_triangle_data), cudaMemcpyHostToDevice)) != cudaSuccess)
-		return cleanup(cuda_fail(e, "upload triangle data"));
-	if ((e = cudaMemset(dStatus, 0, statusBytes)) != cudaSuccess) return cleanup(cuda_fail(e, "clear status"));
-	if (phe_status up = finish_uploads("upload scene")) return cleanup(up);
+		return cuda_fail(e, "upload triangle data");
+	if ((e = cudaMemset(dStatus, 0, statusBytes)) != cudaSuccess) return cuda_fail(e, "clear status");
+	if (phe_status up = finish_uploads("upload scene")) return up;
 
-	phe_scene* sc = new phe_scene();
+	std::unique_ptr<phe_scene, phe_status (*)(phe_scene*)> sc(new phe_scene(), phe_scene_destroy);
 	sc->dev.nodes = dNodes;
 	sc->dev.tris = dTris;
 	sc->dev.datas = dDatas;
@@ -485,17 +490,25 @@ extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNo
 	sc->dev.numTop = numTop;
 	sc->dev.numNodes4 = (uint32_t)(dn4.size() / 8);
 	sc->maxDepth4 = depth4;
-	sc->allocation = base;
+	sc->allocation = allocation.release();
 	sc->bytes = total;
 	sc->status = dStatus;
 	sc->dev.status = dStatus;
 	sc->device = dinfo->device;
-	if (!hm.empty() && (s = upload_shading(sc, hm.data(), (uint32_t)hm.size(), nullptr, 0))) {
-		phe_scene_destroy(sc);
-		return s;
-	}
-	*out = sc;
+	if (!hm.empty() && (s = upload_shading(sc.get(), hm.data(), (uint32_t)hm.size(), nullptr, 0))) return s;
+	*out = sc.release();
 	return PHE_OK;
+}
+
+extern "C" phe_status phe_scene_create(const phe_bvh_node* nodes, uint32_t numNodes, const phe_triangle_vertices* verts,
+                                       const phe_triangle_data* datas, uint32_t numSlots, const phe_material* materials,
+                                       uint32_t numMaterials, int where, phe_scene** out)
+{
+	try {
+		return create_scene(nodes, numNodes, verts, datas, numSlots, materials, numMaterials, where, out);
+	} catch (const std::bad_alloc&) {   // the layout on the host
+		return fail(PHE_ERR_OUT_OF_MEMORY, "phe_scene_create: host allocation failed");
+	}
 }
 
 extern "C" phe_status phe_scene_set_materials_and_textures(phe_scene* scene, const phe_material* materials,

@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -30,6 +31,8 @@ uintptr_t g_handles = 16;      // streams and events are numbers
 std::vector<Launch> g_launches;
 std::vector<std::pair<void*, size_t>> g_allocations;   // in order of allocation
 std::vector<Config> g_configs;
+int g_live = 0;                // allocations not freed
+thread_local long g_newsLeft = -1;   // host allocations until one fails (-1: none does)
 
 std::map<const void*, std::string>& kernel_names()
 {
@@ -48,9 +51,21 @@ cudaError_t record(const void* f, dim3 grid, dim3 block, cudaStream_t s, bool ea
 
 } // namespace
 
+// The library's host allocations, of which one can be made to fail.
+void* operator new(size_t n)
+{
+	if (g_newsLeft >= 0 && g_newsLeft-- == 0) throw std::bad_alloc();
+	if (void* p = std::malloc(n ? n : 1)) return p;
+	throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+
 extern "C" {
 
 // What the tests set and read.
+void fake_fail_new(long after) { g_newsLeft = after; }
+int fake_live_allocations() { return g_live; }
 void fake_set_device(int device) { g_device = device; }
 void fake_set_occupancy(int device, int blocks) { g_occupancy[device] = blocks; }
 int fake_num_launches() { return (int)g_launches.size(); }
@@ -138,9 +153,15 @@ cudaError_t cudaMalloc(void** p, size_t n)
 	if (!*p) return cudaErrorMemoryAllocation;
 	std::memset(*p, 0xCD, size);
 	g_allocations.push_back({*p, n});
+	g_live++;
 	return cudaSuccess;
 }
-cudaError_t cudaFree(void* p) { return std::free(p), cudaSuccess; }
+cudaError_t cudaFree(void* p)
+{
+	g_live -= p != nullptr;
+	std::free(p);
+	return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return *p = std::calloc(1, n), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return std::memcpy(d, s, n), cudaSuccess; }

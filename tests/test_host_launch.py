@@ -43,6 +43,7 @@ def _use(library):
         fn.restype, fn.argtypes = res, args
     lib.fake_allocation.restype = C.c_void_p
     lib.fake_launch.restype = C.c_char_p
+    lib.fake_fail_new.argtypes = [C.c_long]
     native._lib = lib
     return lib
 
@@ -175,3 +176,28 @@ def test_stages_start_early_only_behind_a_kernel(fake_library, schedule, timed, 
     """A frame stage is launched early only where the kernel before it is the stream's last work: not behind the events
     of a timed frame, nor behind the fork and the join of the beside schedule (1)."""
     _in_child(_frame_launches, fake_library, schedule, timed, want)
+
+
+def _upload_without_memory(library):
+    lib = _use(library)
+    s = P.generate_scene(8, 2, False, 7)
+    b = P.build_sbvh(s.tri_verts)
+    P.Scene.from_bvh(b, s).close()   # the device's own allocations are made
+    live = lib.fake_live_allocations()
+    datas, h = b.slot_datas(s.datas), C.c_void_p()
+    for k in range(10000):
+        lib.fake_fail_new(k)
+        st = lib.phe_scene_create(native.ptr(b.nodes), len(b.nodes), native.ptr(b.verts), native.ptr(datas), len(b.verts),
+                                  native.ptr(s.materials), len(s.materials), native.PTR_HOST, C.byref(h))
+        lib.fake_fail_new(-1)
+        if st == native.PHE_OK:
+            break
+        assert st == native.PHE_ERR_OUT_OF_MEMORY and not h.value and lib.fake_live_allocations() == live, (k, st)
+    assert k > 10 and h.value
+    lib.phe_scene_destroy(h)
+    assert lib.fake_live_allocations() == live
+
+
+def test_upload_reports_a_failed_host_allocation(fake_library):
+    """Whichever host allocation fails, the upload returns an error and keeps no device memory."""
+    _in_child(_upload_without_memory, fake_library)
