@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "raygen.cuh"
@@ -647,15 +648,17 @@ resolve_taa_kernel(const FrameParamsDev* __restrict__ fpp, FrameBuffers fb)
 // Without velocities (MOVING false) a texel of the history is read and nothing filtered: 24 registers instead of 44,
 // and as many resident warps again hide the loads: 1920x1080 24.8 us (29.3 with the filtering compiled in), 1280x720 13.2
 // (15.8).
+// HIGH: the image has more rows than a grid's 65,535 blocks along y cover (262,140), and they are split between y and z. An
+// instantiation of its own, since the z index costs the others 0.2% (1920x1080 moving: 34.70 us, 34.62 without).
 constexpr int kTaaBlockX = 32, kTaaBlockY = 4;
-template <bool VEC, bool MOVING>
+template <bool VEC, bool MOVING, bool HIGH>
 __global__ void __launch_bounds__(kTaaBlockX* kTaaBlockY)
 taa_kernel(uint32_t W, uint32_t H, const float4* __restrict__ cur, const float4* __restrict__ hist,
            const float2* __restrict__ vel, const float2* __restrict__ prevVel, const float* __restrict__ roughness,
            float4* __restrict__ outColor, float4* __restrict__ outHist)
 {
 	uint32_t x = blockIdx.x * kTaaBlockX + threadIdx.x;
-	uint32_t y = (blockIdx.z * gridDim.y + blockIdx.y) * kTaaBlockY + threadIdx.y;
+	uint32_t y = (HIGH ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * kTaaBlockY + threadIdx.y;
 	if (x >= W || y >= H) return;
 	size_t p = (size_t)y * W + x;
 	float4 oc, oh;
@@ -839,13 +842,17 @@ extern "C" phe_status phe_taa_resolve(uint32_t resX, uint32_t resY, const float*
 	if (!cur || !hist || !outColor || !outHist) return fail(PHE_ERR_INVALID_ARGUMENT, "phe_taa_resolve: null buffer");
 	if (resX == 0 || resY == 0) return PHE_OK;
 	dim3 block(kTaaBlockX, kTaaBlockY);
-	// A grid has 65,535 blocks along y, 262,140 rows: a higher image's are split between y and z, up to 524,280 rows.
+	// z doubles the blocks along y: up to 524,280 rows.
 	const uint32_t rowBlocks = (resY - 1) / kTaaBlockY + 1, split = rowBlocks > 65535u ? 2u : 1u;
 	dim3 grid((resX - 1) / kTaaBlockX + 1, (rowBlocks - 1) / split + 1, split);
 	// The history and the velocities may be aligned to floats only.
 	const bool vec = !((uintptr_t)hist & 15u) && !((uintptr_t)velocity & 7u) && !((uintptr_t)prevVelocity & 7u);
-	auto kernel = velocity ? (vec ? taa_kernel<true, true> : taa_kernel<false, true>)
-	                       : (vec ? taa_kernel<true, false> : taa_kernel<false, false>);
+	auto pick = [&](auto high) {
+		constexpr bool H = decltype(high)::value;
+		return velocity ? (vec ? taa_kernel<true, true, H> : taa_kernel<false, true, H>)
+		                : (vec ? taa_kernel<true, false, H> : taa_kernel<false, false, H>);
+	};
+	auto kernel = split > 1 ? pick(std::true_type{}) : pick(std::false_type{});
 	kernel<<<grid, block, 0, (cudaStream_t)stream>>>(resX, resY, (const float4*)cur, (const float4*)hist,
 	                                                 (const float2*)velocity, (const float2*)prevVelocity, roughness,
 	                                                 (float4*)outColor, (float4*)outHist);
