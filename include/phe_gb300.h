@@ -258,9 +258,7 @@ phe_status phe_scene_get_layout(const phe_scene* scene, int* layout, int* wideAv
 
 /* OR of error bits raised by kernels on this scene: single casts, frames, batches, no-alloc batches
  * and serving waves (1 = traversal stack overflow, never set for a scene that passed validation;
- * 2 = a node or slot index outside its array, checked build only; 4 = a block's copy of the upper nodes
- * did not arrive in time and it read them from global memory: the results are complete; 8 = that copy was still
- * under way when the block ended, so results of launches at that time may be wrong). Synchronous. */
+ * 2 = a node or slot index outside its array, checked build only). Synchronous. */
 phe_status phe_scene_status(const phe_scene* scene, uint32_t* bits);
 
 /* ---------------------------------------------------------------------------------------------

@@ -59,12 +59,10 @@ struct DeviceScene {
 	const float4* leaves8;  // its leaf records
 	uint32_t numNodes8, numLeaves8;
 	float dirLimit;   // a ray direction with components up to this keeps every |det| below 2^126
-	uint32_t numTop;  // the tree's upper nodes, the first of `nodes` (scene.cu)
+	uint32_t pad2;
 };
 static_assert(sizeof(DeviceScene) == 128, "DeviceScene is 128 bytes");
 
-// Nodes that place_nodes (scene.cu) puts first.
-constexpr uint32_t kTopNodes = 2048;
 constexpr int32_t kEmptyChild = 0x7FFFFFFE;
 
 // Traversal stack depth: leaves of a valid scene are at most 64 levels deep, and a node pushes at
@@ -77,8 +75,6 @@ constexpr int32_t kSentinel = 0x7FFFFFFF;
 // Error bits written to the per-launch status word.
 constexpr uint32_t kErrStackOverflow = 1u;
 constexpr uint32_t kErrBadIndex = 2u;   // checked build: a node or slot index outside its array
-constexpr uint32_t kErrTopCopy = 4u;    // a block's copy of the upper nodes did not arrive in time (it read global memory)
-constexpr uint32_t kErrCopyPending = 8u;   // and had not when the block ended: it may have written another block's shared memory
 
 // The checked build (-DPHE_DEVICE_CHECKS=1, libphe_gb300_checked.so) tests every node and slot index a
 // traversal is about to read against the array sizes; an index outside sets kErrBadIndex and ends that

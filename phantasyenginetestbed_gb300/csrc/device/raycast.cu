@@ -12,7 +12,6 @@
 #include <atomic>
 
 #include "runtime.cuh"
-#include "small_cast.cuh"
 #include "traverse.cuh"
 
 namespace phe_gb300 {
@@ -100,6 +99,34 @@ __global__ void __launch_bounds__(kPersistentBlock, cast_min_blocks(WIDE)) any_p
 	}
 }
 
+// Any hit of few rays: a warp takes 4 to 32 of them, so that fewer lanes wait for one another, and loads three triangles of a
+// leaf at a time, since no other warp hides its loads. (Which rays share a warp changes no answer of an any hit; a closest hit
+// reports the slot of a duplicated triangle that its warp comes to first, and keeps 32 consecutive rays.)
+//
+// Few rays a warp cost instructions that the launches of other streams could issue, so they are taken while the launch makes
+// at most kSmallWarps warps an SM, and a block is one warp without shared memory. 155K triangles, us a cast, this / 32 rays a
+// warp in blocks of 128: 4,096 rays alone 36.9 / 54.9, on 16 streams at once 4.5 / 4.6 (both bound by the host's launches);
+// 8,192 47.7 / 58.9 and 6.2 / 5.9; 16,384 47.8 / 68.3 and 7.2 / 6.8; 40,000 64.2 / 69.6 and 12.4 / 11.9. 4 rays a warp at
+// 16,384: 51.9 alone but 16.9 on 16 streams. The upper nodes copied to shared memory (128 KB a block, one block an SM) made
+// 4,096 closest hits on 10K triangles 45.7 us alone instead of 49.8 and gained nothing on 155K, but launches of several
+// streams waited for one another: on 16 streams 36 us a cast on 155K instead of 5.
+constexpr int kSmallLeaf = 3;
+constexpr uint32_t kSmallWarps = 7, kSmallMaxWarps = 16;   // of a launch, an SM: with fewer than 32 rays each; with 32
+__global__ void __launch_bounds__(32) small_any_kernel(DeviceScene s, const phe_ray_in* __restrict__ rays, uint8_t* __restrict__ inLight,
+                                                       const uint32_t* __restrict__ scatter, uint32_t n, uint32_t raysPerWarp,
+                                                       uint32_t* __restrict__ status)
+{
+	const uint32_t i = blockIdx.x * raysPerWarp + threadIdx.x;
+	if (threadIdx.x >= raysPerWarp || i >= n) return;
+	const RayState r = load_ray(rays, i);
+	HitRecord h = empty_hit(r);
+	const TraversalBounds bd{s.numNodes, s.numSlots};
+	const uint32_t err = fast_ray(r, s.dirLimit) ? traverse<true, true, 0, kSmallLeaf>(s.nodes, s.tris, bd, r, h)
+	                                             : traverse<false, true, 0, kSmallLeaf>(s.nodes, s.tris, bd, r, h);
+	if (err) atomicOr(status, err);
+	inLight[scatter ? __ldg(scatter + i) : i] = h.slot == ~0u ? 1 : 0;
+}
+
 // [closest, any] x [binary, wide]; filled on first use (threads that race store the same value)
 static std::atomic<int> g_persistentBlocksPerSM[4] = {};
 
@@ -128,39 +155,20 @@ static phe_status check_cast_args(const phe_scene* scene, const void* rays, cons
 	return PHE_OK;
 }
 
-// Queues a launch of few rays on binary nodes (*done) or leaves it to the caller.
-//
-// Closest hit keeps 32 consecutive rays a warp: which of a duplicated triangle's slots a ray reports depends on
-// when its warp turns to leaves, so other warps would report other duplicates. Any hit has no such
-// choice and takes as few rays a warp (4 to 32) as fill the resident warps: fewer lanes wait for one another.
-// Where the lines lie (155K triangles, us a call, small / the kernels above): closest hit 4,096 surface rays 75 / 79,
-// 65,536 93 / 96, on 2M triangles 131 / 136 and 233 / 230; any hit 37 / 62 at 4,096, 68 / 76 at the 77,824 rays that
-// 16 warps an SM hold.
-constexpr uint32_t kSmallClosestRays = 49152;
-template <bool ANY>
-static phe_status small_cast(const phe_scene* scene, const phe_ray_in* rays, void* out, const uint32_t* scatter, uint32_t n,
-                             cudaStream_t stream, bool* done)
+// Queues an any-hit launch of few rays on binary nodes (*done) or leaves it to the caller.
+static phe_status small_any(const phe_scene* scene, const phe_ray_in* rays, uint8_t* inLight, const uint32_t* scatter, uint32_t n,
+                            cudaStream_t stream, bool* done)
 {
 	*done = false;
-	if (scene->dev.nodes4 || scene->dev.nodes8 || (!ANY && n > kSmallClosestRays)) return PHE_OK;
+	if (scene->dev.nodes4 || scene->dev.nodes8) return PHE_OK;
 	DeviceInfo* d = nullptr;
 	if (phe_status st = device_info(&d)) return st;
-	const uint32_t maxWarps = (uint32_t)d->numSMs * kSmallMaxWarps;
-	uint32_t perWarp = ANY ? 4u : 32u;
-	while (perWarp < 32u && (n - 1) / perWarp >= maxWarps) perWarp *= 2;
-	if ((n - 1) / perWarp >= maxWarps) return PHE_OK;
-	const uint32_t warps = (n - 1) / perWarp + 1, grid = std::min(warps, (uint32_t)d->numSMs), perBlock = (warps - 1) / grid + 1;
-	const size_t smem = (size_t)scene->dev.numTop * 64u;
-	auto kernel = small_cast_kernel<ANY>;
-	static std::atomic<uint64_t> sized{0};   // devices on which the kernel may use that much shared memory
-	if (!(sized.load(std::memory_order_relaxed) >> d->device & 1u)) {
-		PHE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kTopNodes * 64u)),
-		             "small_cast_kernel shared memory");
-		sized.fetch_or(uint64_t(1) << d->device, std::memory_order_relaxed);
-	}
-	kernel<<<grid, 32 * perBlock, smem, stream>>>(scene->dev, rays, out, scatter, n, scene->dev.numTop, perWarp, kCopyWaits,
-	                                           scene->status);
-	PHE_CUDA_TRY(cudaGetLastError(), "small_cast_kernel launch");
+	uint32_t perWarp = 4;
+	while (perWarp < 32u && (n - 1) / perWarp >= (uint32_t)d->numSMs * kSmallWarps) perWarp *= 2;
+	const uint32_t warps = (n - 1) / perWarp + 1;
+	if (warps > (uint32_t)d->numSMs * kSmallMaxWarps) return PHE_OK;
+	small_any_kernel<<<warps, 32, 0, stream>>>(scene->dev, rays, inLight, scatter, n, perWarp, scene->status);
+	PHE_CUDA_TRY(cudaGetLastError(), "small_any_kernel launch");
 	*done = true;
 	return PHE_OK;
 }
@@ -176,8 +184,6 @@ extern "C" phe_status phe_cast_closest_plain(const phe_scene* scene, const phe_r
 	if (st) return st;
 	if (((uintptr_t)hits & 15u) != 0) return fail(PHE_ERR_INVALID_ARGUMENT, "hit buffer must be 16-byte aligned");
 	if (n == 0) return PHE_OK;
-	bool done = false;
-	if ((st = small_cast<false>(scene, rays, hits, nullptr, n, (cudaStream_t)stream, &done)) || done) return st;
 	uint32_t grid = (n + kPlainBlock - 1) / kPlainBlock;
 	auto kernel = (scene->dev.nodes4 || scene->dev.nodes8) ? closest_plain_kernel<true> : closest_plain_kernel<false>;
 	kernel<<<grid, kPlainBlock, stack_smem_bytes(kPlainBlock), (cudaStream_t)stream>>>(scene->dev, rays, hits, n,
@@ -194,8 +200,6 @@ extern "C" phe_status phe_cast_closest(const phe_scene* scene, const phe_ray_in*
 	if (((uintptr_t)hits & 15u) != 0) return fail(PHE_ERR_INVALID_ARGUMENT, "hit buffer must be 16-byte aligned");
 	if (n == 0) return PHE_OK;
 	if (n > kMaxPersistentRays) return fail(PHE_ERR_TOO_LARGE, "phe_cast_closest: at most %u rays per launch", kMaxPersistentRays);
-	bool done = false;
-	if ((st = small_cast<false>(scene, rays, hits, nullptr, n, (cudaStream_t)stream, &done)) || done) return st;
 	const bool wide = scene->dev.nodes4 || scene->dev.nodes8;
 	auto kernel = wide ? closest_persistent_kernel<true> : closest_persistent_kernel<false>;
 	int grid = 0;
@@ -218,7 +222,7 @@ extern "C" phe_status phe_cast_any(const phe_scene* scene, const phe_ray_in* ray
 	if (n == 0) return PHE_OK;
 	if (n > kMaxPersistentRays) return fail(PHE_ERR_TOO_LARGE, "phe_cast_any: at most %u rays per launch", kMaxPersistentRays);
 	bool done = false;
-	if ((st = small_cast<true>(scene, rays, inLight, scatter, n, (cudaStream_t)stream, &done)) || done) return st;
+	if ((st = small_any(scene, rays, inLight, scatter, n, (cudaStream_t)stream, &done)) || done) return st;
 	const bool wide = scene->dev.nodes4 || scene->dev.nodes8;
 	auto kernel = wide ? any_persistent_kernel<true> : any_persistent_kernel<false>;
 	int grid = 0;

@@ -92,31 +92,14 @@ __device__ __forceinline__ bool visit_packed(const SlabRay& w, f32x2 loxy, f32x2
 struct NodeData {
 	f32x2 lo0, hi0, lo1, hi1, z0, z1, ref, count;
 };
-// Where the binary traversal reads nodes from: global memory, or a copy of the first numTop nodes (the
-// tree's upper levels, scene.cu) in shared memory and the rest in global memory.
-struct GlobalNodes {
-	const float4* __restrict__ nodes;
-	__device__ __forceinline__ NodeData load(int32_t n) const
-	{
-		const float4* p = nodes + 4 * (size_t)n;
-		NodeData d;
-		ld32(p, d.lo0, d.hi0, d.lo1, d.hi1);
-		ld32(p + 2, d.z0, d.z1, d.ref, d.count);
-		return d;
-	}
-};
-struct TopNodes {
-	const float4* __restrict__ nodes;
-	const ulonglong2* top;   // shared memory
-	uint32_t numTop;
-	__device__ __forceinline__ NodeData load(int32_t n) const
-	{
-		if ((uint32_t)n >= numTop) return GlobalNodes{nodes}.load(n);
-		const ulonglong2* p = top + 4 * (size_t)n;
-		const ulonglong2 a = p[0], b = p[1], c = p[2], e = p[3];
-		return NodeData{a.x, a.y, b.x, b.y, c.x, c.y, e.x, e.y};
-	}
-};
+__device__ __forceinline__ NodeData load_node(const float4* __restrict__ nodes, int32_t n)
+{
+	const float4* p = nodes + 4 * (size_t)n;
+	NodeData d;
+	ld32(p, d.lo0, d.hi0, d.lo1, d.hi1);
+	ld32(p + 2, d.z0, d.z1, d.ref, d.count);
+	return d;
+}
 
 // Both children of a binary node: visit rules, entry distances and references.
 template <bool SAFE>
@@ -182,8 +165,8 @@ using TraversalStack = TraversalStackT<kSmemStack>;
 // LEAF: triangles of a leaf loaded together. 1 where other warps hide a load's latency; more where few
 // warps are resident and a leaf would wait for each triangle in turn (slots past the leaf's last are
 // loaded and not tested: kTriPadding keeps them inside the allocation).
-template <bool SAFE, bool ANY, int SN = kSmemStack, int LEAF = 1, class Nodes>
-__device__ __forceinline__ uint32_t traverse(const Nodes& nodes, const float4* __restrict__ tris,
+template <bool SAFE, bool ANY, int SN = kSmemStack, int LEAF = 1>
+__device__ __forceinline__ uint32_t traverse(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                              const TraversalBounds& bd, const RayState& r, HitRecord& hit)
 {
 	const SlabRay w(r);
@@ -208,7 +191,7 @@ __device__ __forceinline__ uint32_t traverse(const Nodes& nodes, const float4* _
 			float tIn0, tIn1;
 			int32_t c0, c1;
 			bool v0, v1;
-			visit_node<SAFE>(nodes.load(nodeAddr), w, r.tMin, hit.t, v0, v1, tIn0, tIn1, c0, c1);
+			visit_node<SAFE>(load_node(nodes, nodeAddr), w, r.tMin, hit.t, v0, v1, tIn0, tIn1, c0, c1);
 			{
 				const bool both = v0 && v1;
 				const bool swp = !ANY && both && tIn1 < tIn0;
@@ -433,9 +416,9 @@ __device__ __forceinline__ uint32_t trace(const DeviceScene& s, const RayState& 
 				return traverse8<ANY>(s.nodes8, s.leaves8, s.tris, Wide8Bounds{s.numNodes8, s.numLeaves8, s.numSlots}, r, hit);
 			if (s.nodes4) return traverse4<ANY>(s.nodes4, s.tris, TraversalBounds{s.numNodes4, s.numSlots}, r, hit);
 		}
-		return traverse<true, ANY, SN>(GlobalNodes{s.nodes}, s.tris, TraversalBounds{s.numNodes, s.numSlots}, r, hit);
+		return traverse<true, ANY, SN>(s.nodes, s.tris, TraversalBounds{s.numNodes, s.numSlots}, r, hit);
 	}
-	return traverse<false, ANY, SN>(GlobalNodes{s.nodes}, s.tris, TraversalBounds{s.numNodes, s.numSlots}, r, hit);
+	return traverse<false, ANY, SN>(s.nodes, s.tris, TraversalBounds{s.numNodes, s.numSlots}, r, hit);
 }
 
 __device__ __forceinline__ void store_hit(phe_ray_hit* __restrict__ hits, uint32_t i, const RayState& r, const HitRecord& h)
@@ -478,7 +461,7 @@ __device__ __forceinline__ void trace_step(const float4* __restrict__ nodes, con
 		float tIn0, tIn1;
 		int32_t c0, c1;
 		bool v0, v1;
-		visit_node<SAFE>(GlobalNodes{nodes}.load(nodeAddr), w, r.tMin, hit.t, v0, v1, tIn0, tIn1, c0, c1);
+		visit_node<SAFE>(load_node(nodes, nodeAddr), w, r.tMin, hit.t, v0, v1, tIn0, tIn1, c0, c1);
 		if (!v0 && !v1) {
 			nodeAddr = stack.get(sp--);
 		} else {

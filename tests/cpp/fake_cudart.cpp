@@ -16,7 +16,7 @@ namespace {
 struct Launch {
 	std::string kernel;
 	dim3 grid, block;
-	cudaStream_t stream;
+	size_t smem;
 	bool early;   // with the programmatic-serialization attribute
 };
 struct Config {
@@ -41,11 +41,11 @@ std::map<const void*, std::string>& kernel_names()
 }
 cudaError_t g_lastError = cudaSuccess;
 
-cudaError_t record(const void* f, dim3 grid, dim3 block, cudaStream_t s, bool early)
+cudaError_t record(const void* f, dim3 grid, dim3 block, size_t smem, bool early)
 {
 	if (!grid.x || !grid.y || !grid.z || grid.x > 0x7FFFFFFFu || grid.y > 65535u || grid.z > 65535u)
 		return g_lastError = cudaErrorInvalidConfiguration;
-	g_launches.push_back({kernel_names()[f], grid, block, s, early});
+	g_launches.push_back({kernel_names()[f], grid, block, smem, early});
 	return cudaSuccess;
 }
 
@@ -69,11 +69,12 @@ int fake_live_allocations() { return g_live; }
 void fake_set_device(int device) { g_device = device; }
 void fake_set_occupancy(int device, int blocks) { g_occupancy[device] = blocks; }
 int fake_num_launches() { return (int)g_launches.size(); }
-const char* fake_launch(int i, uint32_t grid[3], uint32_t block[3], int* early)
+const char* fake_launch(int i, uint32_t grid[3], uint32_t block[3], size_t* smem, int* early)
 {
 	const Launch& l = g_launches[i];
 	grid[0] = l.grid.x, grid[1] = l.grid.y, grid[2] = l.grid.z;
 	block[0] = l.block.x, block[1] = l.block.y, block[2] = l.block.z;
+	*smem = l.smem;
 	*early = l.early;
 	return l.kernel.c_str();
 }
@@ -108,9 +109,9 @@ cudaError_t __cudaGetKernel(void** handle, const void* f)
 	*handle = const_cast<void*>(f);
 	return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(void* handle, dim3 grid, dim3 block, void**, size_t, cudaStream_t s)
+cudaError_t __cudaLaunchKernel(void* handle, dim3 grid, dim3 block, void**, size_t smem, cudaStream_t)
 {
-	return record(handle, grid, block, s, false);
+	return record(handle, grid, block, smem, false);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**)
 {
@@ -118,7 +119,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 	for (unsigned i = 0; i < c->numAttrs; i++)
 		early = early || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
 		                  c->attrs[i].val.programmaticStreamSerializationAllowed);
-	return record(f, c->gridDim, c->blockDim, c->stream, early);
+	return record(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, early);
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t)
 {

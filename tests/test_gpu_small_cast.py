@@ -115,40 +115,3 @@ def test_counter_cleared_in_and_out_of_a_graph(n):
         with torch.cuda.stream(stream):
             graph.replay()
         check()
-
-
-@pytest.fixture(scope="module")
-def small_cast_once(tmp_path_factory):
-    import ctypes as C
-    import subprocess
-    from pathlib import Path
-
-    from phantasyenginetestbed_gb300 import build as B
-    root, lib = Path(__file__).resolve().parents[1], B.build()
-    out = tmp_path_factory.mktemp("small") / "small_cast_test.so"
-    subprocess.run([B._nvcc(), *B.ARCH, "-O3", "-std=c++17", "-fmad=false", "-shared", "-Xcompiler", "-fPIC", f"-I{root / 'include'}",
-                    f"-I{B.CSRC / 'device'}", str(root / "tests/cpp/small_cast_test.cu"), "-o", str(out), f"-L{lib.parent}",
-                    "-lphe_gb300", f"-Xlinker=-rpath,{lib.parent}"], check=True)
-    fn = C.CDLL(str(out)).small_cast_once
-    fn.argtypes = [C.c_void_p] * 4 + [C.c_uint32, C.c_int, C.c_uint32, C.c_uint32]
-    return fn
-
-
-@pytest.mark.parametrize("name", ["c2_256_2000", "one_leaf"])
-@pytest.mark.parametrize("n", [1, 33, 152 * 32 + 1, 9728])
-def test_late_copy_of_the_upper_nodes(small_cast_once, name, n):
-    """A first wait of no tries: every thread reads global memory and says so; the results are the same."""
-    import torch
-    b, _, _, d_rays, hits, vis = _large(name)
-    scene = P.Scene(b.nodes, b.verts)
-    order = np.random.default_rng(n).permutation(n).astype(np.uint32)
-    d_order = to_device(order)
-    for waits, bits in ((1 << 20, 0), (0, 4)):
-        out = device_empty(n, P.RAY_HIT_DTYPE)
-        lit = device_empty(n, np.uint8)
-        assert small_cast_once(scene.handle, d_rays.data_ptr(), out.data_ptr(), None, n, 0, 32, waits) == 0
-        assert small_cast_once(scene.handle, d_rays.data_ptr(), lit.data_ptr(), d_order.data_ptr(), n, 1, 4, waits) == 0
-        torch.cuda.synchronize()
-        assert np.array_equal(from_device(out, np.uint8), hits[:n].view(np.uint8))
-        assert np.array_equal(from_device(lit, np.uint8)[order], vis[:n])
-        assert scene.status() == bits

@@ -55,12 +55,12 @@ def _allocation(lib, i):
 
 
 def _launches(lib):
-    """Every launch so far: kernel, grid, block, whether it may start early."""
+    """Every launch so far: kernel, grid, block, dynamic shared memory, whether it may start early."""
     out = []
     for i in range(lib.fake_num_launches()):
-        grid, block, early = (C.c_uint32 * 3)(), (C.c_uint32 * 3)(), C.c_int()
-        name = lib.fake_launch(i, grid, block, C.byref(early)).decode()
-        out.append((name, tuple(grid), tuple(block), bool(early.value)))
+        grid, block, smem, early = (C.c_uint32 * 3)(), (C.c_uint32 * 3)(), C.c_size_t(), C.c_int()
+        name = lib.fake_launch(i, grid, block, C.byref(smem), C.byref(early)).decode()
+        out.append((name, tuple(grid), tuple(block), smem.value, bool(early.value)))
     return out
 
 
@@ -118,7 +118,7 @@ def _taa_heights(library):
     buf = C.c_void_p(1 << 20)
     for h in (1, 4, 5, 262140, 262141, 262149, 524279, 524280):
         assert lib.phe_taa_resolve(40, h, buf, buf, None, None, None, buf, buf, None) == native.PHE_OK, h
-        name, grid, block, _ = _launches(lib)[-1]
+        name, grid, block, _, _ = _launches(lib)[-1]
         assert "taa_kernel" in name and grid[0] * block[0] >= 40 and grid[1] * grid[2] * block[1] >= h
     n = lib.fake_num_launches()
     assert lib.phe_taa_resolve(40, 524281, buf, buf, None, None, None, buf, buf, None) == native.PHE_ERR_CUDA
@@ -139,7 +139,7 @@ def _batch_grids(library, graph):
         scene = P.Scene(b.nodes, b.verts)
         batch = Batch([scene], [(0, 0, 1 << 20, 1 << 20, 2 << 20), (0, 1, 1 << 20, 3 << 20, 4 << 20)], use_graph=graph)
         batch.launch()
-        name, grid, block, _ = _launches(lib)[-1]
+        name, grid, block, _, _ = _launches(lib)[-1]
         assert "batch_kernel" in name and grid == (152 * blocks, 1, 1) and block[0] == 128, (name, grid)
 
 
@@ -162,7 +162,7 @@ def _frame_launches(library, schedule, timed, want):
     r.updateCamera((0.5, -0.3, 0.6), (0.0, 0.8, -0.6), (0.0, 0.6, 0.8), 60.0)
     n = lib.fake_num_launches()
     r.render(R.make_lights(np.array([[0.1, 0.1, 0.5]], np.float32), range_=100.0))
-    got = [(k, early) for name, _, _, early in _launches(lib)[n:]
+    got = [(k, early) for name, _, _, _, early in _launches(lib)[n:]
            for k in ("primary", "any_queue", "bounce", "resolve_taa") if k + "_kernel" in name]
     assert got == want, got
 
@@ -201,3 +201,20 @@ def _upload_without_memory(library):
 def test_upload_reports_a_failed_host_allocation(fake_library):
     """Whichever host allocation fails, the upload returns an error and keeps no device memory."""
     _in_child(_upload_without_memory, fake_library)
+
+
+def _small_casts(library):
+    lib = _use(library)
+    b = P.build_sbvh(P.generate_scene(64, 100, False, 7).tri_verts)
+    scene, buf = P.Scene(b.nodes, b.verts), 1 << 20
+    for n in (1, 4096, 8192, 49152, 77824, 77825):
+        for cast in (P.cast_closest, P.cast_closest_plain, P.cast_any):
+            cast(scene, buf, buf, n)
+            name, grid, block, smem, _ = _launches(lib)[-1]
+            warps = grid[0] * block[0] // 32
+            assert smem == 0 and block[0] <= 128 and warps <= max((n + 127) // 128 * 4, 152 * 7), (name, grid, block, smem, n)
+
+
+def test_small_casts_leave_room_for_others(fake_library):
+    """A cast of few rays holds no SM for itself: launches of other streams run beside it."""
+    _in_child(_small_casts, fake_library)
