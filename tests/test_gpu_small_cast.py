@@ -115,3 +115,15 @@ def test_counter_cleared_in_and_out_of_a_graph(n):
         with torch.cuda.stream(stream):
             graph.replay()
         check()
+
+
+@pytest.mark.parametrize("n", [k * 152 * 7 + d for k in (4, 8, 16) for d in (0, 1)])
+def test_any_hit_where_the_rays_per_warp_change(n):
+    import torch
+    _, scene, _, d_rays, _, vis = _large("c2_256_2000")
+    order = np.random.default_rng(n).permutation(n).astype(np.uint32)
+    out = torch.full((n + 16,), 7, dtype=torch.uint8, device="cuda")
+    P.cast_any(scene, d_rays, out, n, scatter=to_device(order))
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert np.array_equal(got[:n][order], vis[:n]) and np.all(got[n:] == 7)
