@@ -139,13 +139,15 @@ void place_nodes(const std::vector<phe_bvh_node>& nodes, std::vector<uint32_t>& 
 }
 
 // Largest ray-direction component D for which |det| = |e1 . (d x e2)| <= 6 D E^2 stays below 2^126 (E: the
-// largest edge component, as the bits of its magnitude), with a factor of four to spare for rounding; -1 (no
-// direction) when an edge is not finite.
+// largest finite edge component, as the bits of its magnitude), with a factor of four to spare for rounding.
+//
+// A triangle with an edge that is not finite does not count: with either reciprocal no ray hits it. A component that is not
+// finite makes two components of its cross product so (a product with 0 is NaN), and then det and one of e2 . r's factors:
+// neither det nor e2 . r is finite. So f is 0 or NaN, t = f (e2 . r) is NaN, and tMin <= t fails.
 float direction_limit(uint32_t largestEdgeBits)
 {
 	float e;
 	std::memcpy(&e, &largestEdgeBits, sizeof(e));
-	if (!std::isfinite(e)) return -1.0f;
 	const double limit = 0x1p124 / (6.0 * (double)e * (double)e);
 	return (float)std::min(limit, (double)3.402823466e+38f);
 }
@@ -378,7 +380,7 @@ static phe_status create_scene(const phe_bvh_node* nodes, uint32_t numNodes, con
 		int4 iv = make_int4(idx[0], idx[1], cnt[0], cnt[1]);
 		std::memcpy(&o[3], &iv, sizeof(iv));
 	}
-	uint32_t largestEdge = 0;   // of the edges' components, the bits of the magnitude (NaN above infinity above the rest)
+	uint32_t largestEdge = 0;   // of the components of triangles whose edges are finite, the bits of the magnitude
 	for (uint32_t i = 0; i < numSlots; i++) {
 		const phe_triangle_vertices& t = hv[i];
 		float e1x = t.v1[0] - t.v0[0], e1y = t.v1[1] - t.v0[1], e1z = t.v1[2] - t.v0[2];
@@ -389,7 +391,9 @@ static phe_status create_scene(const phe_bvh_node* nodes, uint32_t numNodes, con
 		o[2] = make_float4(e2z, e1z, 0.0f, 0.0f);
 		uint32_t edges[6];
 		std::memcpy(edges, &o[1], sizeof(edges));
-		for (uint32_t x : edges) largestEdge = std::max(largestEdge, x & 0x7FFFFFFFu);
+		uint32_t largest = 0;   // NaN above infinity above the rest
+		for (uint32_t x : edges) largest = std::max(largest, x & 0x7FFFFFFFu);
+		if (largest < 0x7F800000u) largestEdge = std::max(largestEdge, largest);
 	}
 	// End markers from the leaf ranges of the reachable tree (phe_bvh_validate checked the ranges).
 	{

@@ -17,6 +17,7 @@ struct Launch {
 	std::string kernel;
 	dim3 grid, block;
 	size_t smem;
+	std::string scene;   // the bytes of a scene passed by value as the first argument
 	bool early;   // with the programmatic-serialization attribute
 };
 struct Config {
@@ -41,11 +42,13 @@ std::map<const void*, std::string>& kernel_names()
 }
 cudaError_t g_lastError = cudaSuccess;
 
-cudaError_t record(const void* f, dim3 grid, dim3 block, size_t smem, bool early)
+cudaError_t record(const void* f, dim3 grid, dim3 block, size_t smem, void** args, bool early)
 {
 	if (!grid.x || !grid.y || !grid.z || grid.x > 0x7FFFFFFFu || grid.y > 65535u || grid.z > 65535u)
 		return g_lastError = cudaErrorInvalidConfiguration;
-	g_launches.push_back({kernel_names()[f], grid, block, smem, early});
+	const std::string& name = kernel_names()[f];
+	const bool scene = name.find("EvNS_11DeviceScene") != std::string::npos;
+	g_launches.push_back({name, grid, block, smem, scene ? std::string((const char*)args[0], 128) : "", early});
 	return cudaSuccess;
 }
 
@@ -78,6 +81,7 @@ const char* fake_launch(int i, uint32_t grid[3], uint32_t block[3], size_t* smem
 	*early = l.early;
 	return l.kernel.c_str();
 }
+const char* fake_launch_scene(int i) { return g_launches[i].scene.size() == 128 ? g_launches[i].scene.data() : nullptr; }
 int fake_num_allocations() { return (int)g_allocations.size(); }
 void* fake_allocation(int i, size_t* bytes)
 {
@@ -109,17 +113,17 @@ cudaError_t __cudaGetKernel(void** handle, const void* f)
 	*handle = const_cast<void*>(f);
 	return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(void* handle, dim3 grid, dim3 block, void**, size_t smem, cudaStream_t)
+cudaError_t __cudaLaunchKernel(void* handle, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t)
 {
-	return record(handle, grid, block, smem, false);
+	return record(handle, grid, block, smem, args, false);
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**)
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args)
 {
 	bool early = false;
 	for (unsigned i = 0; i < c->numAttrs; i++)
 		early = early || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
 		                  c->attrs[i].val.programmaticStreamSerializationAllowed);
-	return record(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, early);
+	return record(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, args, early);
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t)
 {

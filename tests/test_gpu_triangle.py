@@ -61,3 +61,35 @@ def test_long_directions_on_large_scenes(scene_exp, dir_exp):
     assert scene.status() == 0
     if scene_exp == 0 and dir_exp == 0:
         assert (orc["triangleIndex"] != 0xFFFFFFFF).sum() > 1000
+
+
+def test_triangles_with_an_edge_that_is_not_finite():
+    """Vertices at infinity and NaN in a quarter of the slots: their triangles are never hit, as in the oracle, and the
+    rays of the scene take the fast path in every layout."""
+    import torch
+    s = P.generate_scene(24, 20, True, 5)
+    b = P.build_sbvh(s.tri_verts)
+    verts = b.verts.copy()
+    rng = np.random.default_rng(3)
+    for i in rng.permutation(len(verts))[:len(verts) // 4]:
+        verts[("v0", "v1", "v2")[rng.integers(3)]][i, rng.integers(3)] = (np.inf, -np.inf, np.nan)[rng.integers(3)]
+    k = s.scale
+    rays = random_rays(60011, [0, 0, 0.02 * k], [k, k, 0.3 * k], 9, tmin=0.0)
+    rays["dir"][::5, 2] = 0.0   # products of 0 and infinity
+    d_rays = to_device(rays)
+    orc = O.cast_rays(b.nodes, verts, rays, mode=O.MODE_GPU)
+    lit = O.any_rays(b.nodes, verts, rays)
+    slots = orc["triangleIndex"][orc["triangleIndex"] != 0xFFFFFFFF]
+    assert len(slots) > 1000 and all(np.isfinite(verts[f][slots, :3]).all() for f in ("v0", "v1", "v2"))
+    scene = P.Scene(b.nodes, verts)
+    for layout in range(3):
+        scene.set_layout(layout)
+        for n in (1001, len(rays)):
+            hits, vis = device_empty(n, P.RAY_HIT_DTYPE), device_empty(n, np.uint8)
+            P.cast_closest(scene, d_rays, hits, n)
+            P.cast_any(scene, d_rays, vis, n)
+            torch.cuda.synchronize()
+            rep = O.compare_closest(from_device(hits, P.RAY_HIT_DTYPE), orc[:n], rays[:n], b.slot_to_tri, verts)
+            assert rep["ok"] and rep["near_ties"] <= 2, rep
+            assert np.array_equal(from_device(vis, np.uint8), lit[:n])
+    assert scene.status() == 0

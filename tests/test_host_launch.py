@@ -43,6 +43,7 @@ def _use(library):
         fn.restype, fn.argtypes = res, args
     lib.fake_allocation.restype = C.c_void_p
     lib.fake_launch.restype = C.c_char_p
+    lib.fake_launch_scene.restype = C.c_void_p
     lib.fake_fail_new.argtypes = [C.c_long]
     native._lib = lib
     return lib
@@ -218,3 +219,31 @@ def _small_casts(library):
 def test_small_casts_leave_room_for_others(fake_library):
     """A cast of few rays holds no SM for itself: launches of other streams run beside it."""
     _in_child(_small_casts, fake_library)
+
+
+def _direction_limit(library):
+    lib = _use(library)
+    b = P.build_sbvh(P.generate_scene(8, 2, False, 7).tri_verts * np.float32(1024))   # edges long enough for a finite bound
+
+    def limit(verts):
+        scene = P.Scene(b.nodes, verts)
+        P.cast_closest(scene, 1 << 20, 1 << 20, 1000)
+        s = C.string_at(lib.fake_launch_scene(lib.fake_num_launches() - 1), 128)
+        scene.close()
+        return np.frombuffer(s, np.float32)[30]
+
+    want = limit(b.verts)
+    edge = max(np.abs(b.verts[k][:, :3] - b.verts["v0"][:, :3]).max() for k in ("v1", "v2"))
+    assert np.isclose(want, 2.0**124 / (6.0 * np.float64(edge)**2), rtol=1e-6)
+    for k, value in (("v0", np.nan), ("v1", np.inf), ("v2", -np.inf)):
+        v = b.verts.copy()
+        v[k][len(v) // 2, 1] = value
+        assert limit(v) == want
+    v = b.verts.copy()
+    v["v1"][0, 2] = 3e38
+    assert 0 < limit(v) < 1
+
+
+def test_direction_limit_of_a_scene(fake_library):
+    """The bound below which rays take the fast triangle test: from the finite edges alone."""
+    _in_child(_direction_limit, fake_library)
