@@ -257,8 +257,8 @@ phe_status phe_scene_set_layout(phe_scene* scene, int layout);
 phe_status phe_scene_get_layout(const phe_scene* scene, int* layout, int* wideAvailable);
 
 /* OR of error bits raised by kernels on this scene: single casts, frames, batches, no-alloc batches
- * and serving waves (1 = traversal stack overflow, never set for a scene that passed validation;
- * 2 = a node or slot index outside its array, checked build only). Synchronous. */
+ * and serving waves (1 = traversal stack overflow, which no scene that passed validation reaches: the checked build
+ * and the wide layouts test it; 2 = a node or slot index outside its array, checked build only). Synchronous. */
 phe_status phe_scene_status(const phe_scene* scene, uint32_t* bits);
 
 /* ---------------------------------------------------------------------------------------------

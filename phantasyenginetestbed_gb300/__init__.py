@@ -222,7 +222,8 @@ class Scene:
 
     def status(self) -> int:
         """Error bits raised by kernels on this scene so far (1 = traversal stack overflow, 2 = index
-        outside its array, which only the checked build tests); 0 when every traversal was sound."""
+        outside its array; the checked build tests both, the wide layouts the first); 0 when every traversal was
+        sound."""
         bits = C.c_uint32()
         check(lib().phe_scene_status(self.handle, C.byref(bits)), "phe_scene_status")
         return int(bits.value)

@@ -51,8 +51,8 @@ __device__ __forceinline__ uint32_t find_item(const BatchItemDev* __restrict__ i
 // uneven-batch mix over 10K..2M-triangle scenes 2.553 ms vs 2.617 ms with the compiler's own budget
 // (48-56 registers), and 2.932 ms at 40 registers (spills); the autotuner then picks the resident
 // blocks below that limit.
-// Traversal errors (stack overflow; an index outside its array in the checked build) are ORed into the
-// status word of the item's scene, which phe_scene_status reads.
+// Traversal errors (an index outside its array or a full stack, which the checked build tests) are ORed into the status
+// word of the item's scene, which phe_scene_status reads.
 constexpr int kBatchThreadsPerSM = 1280;
 template <int BLOCK, bool WIDE, int SN>
 __global__ void __launch_bounds__(BLOCK, (WIDE ? 128 * kWideMinBlocks : kBatchThreadsPerSM) / BLOCK) batch_kernel(BatchTableDev t, uint32_t* __restrict__ counter)

@@ -13,7 +13,7 @@ constexpr float kU2WhiteInv = 1.0f / kU2White;
 
 // n / d rounded to nearest, for |n|, |d| and the quotient far from the ends of the exponent range: the
 // quotient's approximation n * r corrected with its fused residual (Markstein, IBM J. Res. Dev. 34, 1990), r the
-// rounded reciprocal of d. The compiler's division also guards the ends, with a branch.
+// rounded reciprocal of d.
 __device__ __forceinline__ float divide_in_range(float n, float d, float r)
 {
 	const float q = __fmul_rn(n, r);

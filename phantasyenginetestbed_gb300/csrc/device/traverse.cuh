@@ -160,7 +160,8 @@ struct TraversalStackT {
 using TraversalStack = TraversalStackT<kSmemStack>;
 
 // Traverses the scene for one ray. ANY = true stops at the first triangle with tMin <= t < tMax.
-// Returns the error bits (0, or kErrStackOverflow when the stack would overflow).
+// Returns the error bits of the checked build, else 0: a tree that passed validation is at most 64 levels deep, which
+// the stack holds, so its overflow is tested there only.
 //
 // LEAF: triangles of a leaf loaded together. 1 where other warps hide a load's latency; more where few
 // warps are resident and a leaf would wait for each triangle in turn (slots past the leaf's last are

@@ -510,7 +510,8 @@ __device__ __forceinline__ void taa_blend(float4 cur, float4 h, float trust, flo
 
 // Every texel a moving pixel reads (history and previous velocity around the reprojected position) is
 // requested before the first is used, each as one 8- or 16-byte load: 1080p alone 37 -> 34 us (16.7 M
-// instead of 24.3 M warp instructions); 126 MB of DRAM traffic, bound by its latency behind the velocity.
+// instead of 24.3 M warp instructions); 126 MB of DRAM traffic, 54% of the copy rate: bound by the latency of the gathers
+// behind the velocity.
 template <bool VEC>
 __device__ __forceinline__ void taa_pixel(uint32_t x, uint32_t y, uint32_t W, uint32_t H, float4 cur,
                                           const float4* __restrict__ hist, const float2* __restrict__ vel,
